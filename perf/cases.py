@@ -171,7 +171,8 @@ def _wrap(tensor):
     """A torch tensor's values in a tensor of the framework's."""
     kind = {torch.float32: "F32", torch.bfloat16: "BF16", torch.float16: "F16"}[tensor.dtype]
     mine = llaisys.Tensor(tuple(tensor.shape), llaisys.DataType[kind], llaisys.DeviceType.NVIDIA)
-    mine.load(tensor.cpu())
+    host = tensor.cpu()  # (load() takes an address)
+    mine.load(host)
     return mine
 
 
