@@ -218,6 +218,9 @@ void attention_generic(stream_t stream, llaisysDataType_t dtype, const KVView &k
                    "attention: V rows must have 1 to 1024 elements, K rows at most 8192");
     CHECK_ARGUMENT(kv.nkvh > 0 && batch.nh % kv.nkvh == 0, "attention: nh must be a multiple of nkvh");
     CHECK_ARGUMENT(batch.nh <= 65535, "attention: too many heads for one launch");
+    if (attention_generic_tiles(stream, dtype, kv, batch, q, scale, out)) {
+        return;
+    }
     auto s = static_cast<cudaStream_t>(stream);
     switch (dtype) {
     case LLAISYS_DTYPE_F32:

@@ -191,6 +191,10 @@ void paged_gather(stream_t stream, size_t elem_size, const KVView &kv, int32_t s
 // operator for shapes they do not cover.
 void attention_generic(stream_t stream, llaisysDataType_t dtype, const KVView &kv, const AttnBatch &batch,
                        const void *q, float scale, const AttnOut &out, int32_t *error_flag);
+// Its form for one sequence over plain K/V tensors with head_dim 64 or 128 and the causal mask alone: tiles of rows, keys split over a
+// cluster. False = call not covered, nothing launched (attention_generic then takes its other kernel).
+bool attention_generic_tiles(stream_t stream, llaisysDataType_t dtype, const KVView &kv, const AttnBatch &batch, const void *q, float scale,
+                             const AttnOut &out);
 
 // Attention without a softmax whose weights are mixed over the heads (see GateArgs). Any dtype and sizes, windows but no kept
 // tokens, neither partial results nor output factors. The kernel behind shapes that attention_gates_tiles does not cover.

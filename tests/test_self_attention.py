@@ -98,3 +98,33 @@ def test_multi_token_queries_over_plain_tensors_nvidia(cuda_device, qlen, kvlen,
     f64 = attention.self_attention_f64(q, k, v, scale)
     ulp = {"f16": 1e-3, "bf16": 8e-3}[dname]
     assert helpers.max_abs(got, f64) <= ulp * max(1.0, f64.abs().max().item())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dname", ["f32", "f16", "bf16"])
+@pytest.mark.parametrize("qlen,kvlen,nh,nkvh,d", [
+    (1, 1, 12, 2, 64), (1, 129, 12, 2, 128), (2, 128, 12, 2, 128), (15, 127, 5, 1, 128), (15, 900, 18, 2, 128),  # tiles of 16 rows
+    (65, 65, 32, 8, 64), (86, 300, 12, 2, 64), (96, 777, 12, 2, 128), (300, 301, 12, 2, 64), (257, 513, 33, 3, 128)])  # tiles of 64 rows
+def test_tiles_over_plain_tensors_nvidia(cuda_device, qlen, kvlen, nh, nkvh, d, dname):
+    """Calls that neither 16-bit kernel takes: tiles that end inside the rows, key blocks that end inside a split, groups that do not
+    divide a tile, CTAs of a cluster without keys. A sum of n products in f32 is off by at most n rounding errors of its terms' magnitudes;
+    a softmax row's weights sum to one, so 2 (d + kvlen) x 2^-24 of the largest value bounds scores and outputs."""
+    g = torch.Generator().manual_seed(qlen * kvlen)
+    q, k, v = (workloads.randn((n, h, d), helpers.TORCH_DTYPE[dname], g) for n, h in ((qlen, nh), (kvlen, nkvh), (kvlen, nkvh)))
+    got = helpers.run_self_attention(q, k, v, d ** -0.5, llaisys.DeviceType.NVIDIA, dname)
+    f64 = attention.self_attention_f64(q, k, v, d ** -0.5)
+    rounding = {"f32": 0.0, "f16": 2.0 ** -11, "bf16": 2.0 ** -8}[dname]
+    assert helpers.max_abs(got, f64) <= 2 * (d + kvlen) * 2.0 ** -24 * v.abs().max().item() + rounding * f64.abs().max().item()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("qlen", [3, 96])
+def test_values_behind_the_mask_stay_out_nvidia(cuda_device, qlen, bad):
+    """The last key's V row is not finite: only the last query sees it."""
+    g = torch.Generator().manual_seed(qlen)
+    q, k, v = (workloads.randn((n, h, 128), torch.float32, g) for n, h in ((qlen, 12), (200, 2), (200, 2)))
+    v[-1] = bad
+    got = helpers.run_self_attention(q, k, v, 128 ** -0.5, llaisys.DeviceType.NVIDIA, "f32")
+    assert torch.isfinite(got[:-1]).all() and not torch.isfinite(got[-1]).any()
+    assert helpers.max_abs(got[:-1], attention.self_attention_f64(q[:-1], k[:-1], v[:-1], 128 ** -0.5)) <= 1e-5
