@@ -42,9 +42,17 @@ void linear(stream_t stream, llaisysDataType_t dtype, void *out, const void *in,
 // clears) the kernel's error word: 0, or 16 when a bounded wait ran out.
 // 0 = the streaming kernel where it measured faster (default), 1 = wherever it applies, 2 = never. False: unknown value.
 bool set_linear_policy(int policy);
+int linear_policy();
+// One row x [k] of 16-bit activations: out = f(x) . W^T with f = rms_norm(., gain) or, gain null, nothing; stored, added to out, or (kGlu: W is
+// a packed gate|up matrix of 2 n rows) up * silu(gate). Launched programmatically: W must not be written by the kernel in front. False = not
+// covered (f32, K not a multiple of 8 or over 12000, unaligned, a policy other than 0), nothing launched.
+enum class RowOut { kStore, kAdd, kGlu };
+bool linear_row(stream_t stream, llaisysDataType_t dtype, void *out, const void *x, const void *gain, float eps, const void *weight, size_t n,
+                size_t k, RowOut form);
 bool linear_tc(stream_t stream, llaisysDataType_t dtype, void *out, const void *in, const void *weight, size_t m, size_t n,
                size_t k, bool accumulate, bool overlap);
 int linear_tc_status(stream_t stream);
+int32_t *linear_tc_error_word(); // on the current device
 // out[r, i] = up * silu(gate) with gate = gu[r, i], up = gu[r, di + i]: the activation on a packed gate|up projection.
 void swiglu_packed(stream_t stream, llaisysDataType_t dtype, void *out, const void *gate_up, size_t rows, size_t di);
 // out[r, i] = up * max(gate, 0), packed alike

@@ -111,6 +111,8 @@ bool set_linear_policy(int policy) {
     return true;
 }
 
+int linear_policy() { return g_linear_policy.load(std::memory_order_relaxed); }
+
 void linear(stream_t stream, llaisysDataType_t dtype, void *out, const void *in, const void *weight, const void *bias,
             size_t m, size_t n, size_t k, bool accumulate, size_t in_stride, size_t out_stride) {
     if (m == 0 || n == 0) {

@@ -444,6 +444,8 @@ bool linear_tc(stream_t stream, llaisysDataType_t dtype, void *out, const void *
     return true;
 }
 
+int32_t *linear_tc_error_word() { return gemm_error_word(); }
+
 int linear_tc_status(stream_t stream) {
     int32_t *w = gemm_error_word();
     int32_t host = 0;

@@ -161,6 +161,16 @@ void Qwen2::opLinear(void *out, const void *in, const void *w, size_t m, size_t 
     QWEN2_DISPATCH(cpu::linear(_meta.dtype, out, in, w, nullptr, m, n, k, accumulate),
                    kernels::linear(_stream, _meta.dtype, out, in, w, nullptr, m, n, k, accumulate));
 }
+// One row (a single user's token) takes the norm, the projection and what follows it in one launch; false: not covered, nothing done.
+bool Qwen2::opLinearRow(void *out, const void *in, const void *gain, const void *w, size_t m, size_t n, size_t k, Row form) {
+#ifdef ENABLE_NVIDIA_API
+    if (_on_gpu && m == 1) {
+        const auto f = form == Row::kGlu ? kernels::RowOut::kGlu : form == Row::kAdd ? kernels::RowOut::kAdd : kernels::RowOut::kStore;
+        return kernels::linear_row(_stream, _meta.dtype, out, in, gain, _meta.epsilon, w, n, k, f);
+    }
+#endif
+    return false;
+}
 void Qwen2::opRmsNorm(void *out, const void *in, const void *w, size_t rows, size_t d) {
     QWEN2_DISPATCH(cpu::rms_norm(_meta.dtype, out, in, w, _meta.epsilon, rows, d),
                    kernels::rms_norm(_stream, _meta.dtype, out, in, w, _meta.epsilon, rows, d));
@@ -182,7 +192,9 @@ void Qwen2::setCollective(std::unique_ptr<comm::Collective> c) {
 
 void Qwen2::projectIntoStream(void *x, void *tmp, const void *in, const void *w, size_t m, size_t n, size_t k) {
     if (_tp_world == 1) {
-        opLinear(x, in, w, m, n, k, true); // the residual add folded into the projection
+        if (!opLinearRow(x, in, nullptr, w, m, n, k, Row::kAdd)) {
+            opLinear(x, in, w, m, n, k, true); // the residual add folded into the projection
+        }
         return;
     }
     if (!_tp) {
@@ -213,8 +225,10 @@ void Qwen2::forward(const StepArrays &a, const StepShape &s) {
     opEmbedding(x, a.tokens, _weights.in_embed->tensor->data(), T, hs, _meta.voc);
     for (size_t l = 0; l < _meta.nlayer; ++l) {
         const Layer &w = layers[l];
-        opRmsNorm(h, x, w.attn_norm, T, hs);
-        opLinear(qkv, h, w.qkv_w, T, qd + 2 * kd, hs);
+        if (!opLinearRow(qkv, x, w.attn_norm, w.qkv_w, T, qd + 2 * kd, hs, Row::kStore)) {
+            opRmsNorm(h, x, w.attn_norm, T, hs);
+            opLinear(qkv, h, w.qkv_w, T, qd + 2 * kd, hs);
+        }
         _cache->ropeAppendDev(l, q, qkv, w.qkv_b, a.seq32, a.pos32, T, _meta.nh, _meta.theta, _stream);
         if (s.decode_only) {
             _cache->decodeDev(l, attn, nullptr, q, a.seq_list, a.kv_lens, n_seqs, s.max_kv_len, _meta.nh, scale, _stream);
@@ -223,9 +237,11 @@ void Qwen2::forward(const StepArrays &a, const StepShape &s) {
                                scale, _stream);
         }
         projectIntoStream(x, h, attn, w.o_w, T, hs, qd);
-        opRmsNorm(h, x, w.mlp_norm, T, hs);
-        opLinear(gate_up, h, w.gate_up_w, T, 2 * di, hs);
-        opSwigluPacked(act, gate_up, T, di);
+        if (!opLinearRow(act, x, w.mlp_norm, w.gate_up_w, T, di, hs, Row::kGlu)) {
+            opRmsNorm(h, x, w.mlp_norm, T, hs);
+            opLinear(gate_up, h, w.gate_up_w, T, 2 * di, hs);
+            opSwigluPacked(act, gate_up, T, di);
+        }
         projectIntoStream(x, h, act, w.down_w, T, hs, di);
     }
     if (s.n_out == 0) {
@@ -237,8 +253,11 @@ void Qwen2::forward(const StepArrays &a, const StepShape &s) {
         opEmbedding(_x_last->memory(), a.out_rows, x, s.n_out, hs, T);
         last = _x_last->memory();
     }
-    opRmsNorm(_x_last->memory(), last, _weights.out_norm_w->tensor->data(), s.n_out, hs);
-    opLinear(_logits->memory(), _x_last->memory(), _weights.out_embed->tensor->data(), s.n_out, _meta.voc, hs);
+    if (!opLinearRow(_logits->memory(), last, _weights.out_norm_w->tensor->data(), _weights.out_embed->tensor->data(), s.n_out, _meta.voc, hs,
+                     Row::kStore)) {
+        opRmsNorm(_x_last->memory(), last, _weights.out_norm_w->tensor->data(), s.n_out, hs);
+        opLinear(_logits->memory(), _x_last->memory(), _weights.out_embed->tensor->data(), s.n_out, _meta.voc, hs);
+    }
     opArgmax(a.next, _logits->memory(), s.n_out, _meta.voc);
 }
 

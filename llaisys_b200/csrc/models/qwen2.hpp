@@ -48,6 +48,8 @@ private:
     // operator shims: CPU loops or CUDA launches on the runtime stream, on raw device pointers
     void opEmbedding(void *out, const int64_t *idx, const void *w, size_t n, size_t d, size_t vocab);
     void opLinear(void *out, const void *in, const void *w, size_t m, size_t n, size_t k, bool accumulate = false);
+    enum class Row { kStore, kAdd, kGlu };
+    bool opLinearRow(void *out, const void *in, const void *gain, const void *w, size_t m, size_t n, size_t k, Row form);
     void opRmsNorm(void *out, const void *in, const void *w, size_t rows, size_t d);
     void opSwigluPacked(void *out, const void *gate_up, size_t rows, size_t di);
     void opAdd(void *c, const void *a, const void *b, size_t n);

@@ -248,3 +248,30 @@ def test_cached_step_graph_survives_a_first_prefill_nvidia():
         for pos in range(len(h) - 1):
             row = rows[pos]
             assert (row.max() - row[h[pos + 1]]).item() <= 2 * tol * max(1.0, row.abs().max().item()), (h, pos)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["bf16", "f16"])
+@pytest.mark.parametrize("hidden,inter,vocab", [(256, 512, 321), (264, 6400, 320), (1536, 200, 1001), (512, 12008, 64), (256, 36, 320)])
+def test_single_rows_take_one_launch_per_projection_nvidia(cuda_device, dtype, hidden, inter, vocab):
+    """One token of one sequence runs norm + projection + what follows in single launches: depths that one warp and that eight warps share,
+    odd output counts, a depth past the kernel's bound and one that is not made of 16-byte pieces (general path). The logits after several
+    steps lie no further from the f32 model than those of the general path, give or take the two paths' rounding."""
+    kind, t = (llaisys.DataType.BF16, torch.bfloat16) if dtype == "bf16" else (llaisys.DataType.F16, torch.float16)
+    cfg, hf = hf_model(seed=3, std=0.03, hidden_size=hidden, intermediate_size=inter, vocab_size=vocab, head_dim=128)
+    hf = hf.to(t).float()  # the rounded weights, in f32
+    prompt = np.random.default_rng(hidden).integers(0, min(vocab, 300), 21).tolist()
+    want = hf_logits(hf, prompt)[-1]
+    off = {}
+    for policy in (0, 2):
+        llaisys.Ops.set_linear_policy(policy)
+        try:
+            model = make(cfg, hf.to(t), llaisys.DeviceType.NVIDIA, kind)
+            seq = model.add_seq() if model.configure_cache(1, 64) is None else -1
+            for token in prompt:  # (the first steps run eagerly, the later ones as a graph)
+                model.step([seq], [[token]])
+            off[policy] = (torch.from_numpy(model.last_logits()[0]) - want).norm().item() / want.norm().item()
+            hf = hf.float()
+        finally:
+            llaisys.Ops.set_linear_policy(0)
+    assert off[0] <= 1.5 * off[2] + {"bf16": 2 ** -8, "f16": 2 ** -11}[dtype], off
