@@ -94,6 +94,7 @@ public:
     int lastKernel() const { return _last_kernel; }
     void flush(); // queue uploads of the table rows that changed since the last flush
     void check(); // synchronise, throw LLAISYS_E_KERNEL if a kernel flagged bad metadata
+    const void *errorWord() const { return _error_dev->memory(); } // on the device; check() reads, reports and clears it
 
     // ---- data path: host index arrays (validated, staged, queued on the calling thread's stream) ----
     void append(size_t layer, const void *k_rows, const void *v_rows, const int32_t *seq_ids, const int32_t *positions,

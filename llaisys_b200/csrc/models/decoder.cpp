@@ -33,6 +33,7 @@ Decoder::Decoder(const char *name, llaisysDeviceType_t device, int device_id, ll
 
 Decoder::~Decoder() {
     dropStepGraphs();
+    freeResults();
     for (ModelObserver *o : std::vector<ModelObserver *>(_observers)) {
         o->modelDestroyed();
     }
@@ -261,6 +262,46 @@ void Decoder::copyToHost(void *dst, const void *src, size_t bytes) {
     }
 }
 
+// A step's results and the kernels' error words behind ONE synchronisation (each by itself cost a step 15 us); true: a word is set.
+bool Decoder::copyResults(void *dst, const void *src, size_t bytes) {
+    auto &rt = enter();
+#ifdef ENABLE_NVIDIA_API
+    if (_on_gpu) {
+        const size_t words_at = align_up(bytes, 16), need = words_at + 16;
+        if (need > _results_bytes) {
+            freeResults();
+            _results = static_cast<std::byte *>(rt.api()->malloc_host(need * 2));
+            _results_bytes = _results != nullptr ? need * 2 : 0;
+        }
+        if (_results != nullptr) {
+            auto *words = reinterpret_cast<int32_t *>(_results + words_at);
+            if (bytes != 0) {
+                rt.api()->memcpy_async(_results, src, bytes, LLAISYS_MEMCPY_D2H, _stream);
+            }
+            rt.api()->memcpy_async(words, _cache->errorWord(), sizeof(int32_t), LLAISYS_MEMCPY_D2H, _stream);
+            rt.api()->memcpy_async(words + 1, kernels::linear_tc_error_word(), sizeof(int32_t), LLAISYS_MEMCPY_D2H, _stream);
+            rt.synchronize();
+            if (bytes != 0) {
+                std::memcpy(dst, _results, bytes);
+            }
+            return words[0] != 0 || words[1] != 0;
+        }
+    }
+#endif
+    if (bytes != 0) {
+        copyToHost(dst, src, bytes);
+    }
+    return true; // (checkKernels looks at the words itself)
+}
+
+void Decoder::freeResults() {
+    if (_results != nullptr) {
+        enter().api()->free_host(_results);
+        _results = nullptr;
+        _results_bytes = 0;
+    }
+}
+
 // ---- steps ------------------------------------------------------------------------------------------------------------
 
 void Decoder::step(const int32_t *seq_ids, const int32_t *n_tokens, size_t n_seqs, const int64_t *tokens, int64_t *next_out) {
@@ -397,15 +438,15 @@ void Decoder::stepRows(const int32_t *seq_ids, const int32_t *n_tokens, size_t n
         forward(a, shape);
     }
     _last_n_out = n_rows;
-    if (n_rows != 0) {
-        copyToHost(next_out, a.next, n_rows * sizeof(int64_t));
-    }
+    const bool flagged = copyResults(next_out, a.next, n_rows * sizeof(int64_t));
     for (size_t i = 0, at = 0; i < n_seqs; ++i) {
         seqLen(seq_ids[i]) += size_t(n_tokens[i]);
         recordTokens(seq_ids[i], tokens + at, size_t(n_tokens[i]));
         at += size_t(n_tokens[i]);
     }
-    checkKernels();
+    if (flagged) {
+        checkKernels();
+    }
 }
 
 void Decoder::decodeLoop(const int32_t *seq_ids, size_t n_seqs, const int64_t *first_tokens, size_t n_steps,
@@ -522,7 +563,7 @@ void Decoder::decodeLoop(const int32_t *seq_ids, size_t n_seqs, const int64_t *f
         _last_loop_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count() / double(n_steps);
     }
     _last_n_out = n_seqs;
-    copyToHost(tokens_out, log_dev, n_steps * n_seqs * sizeof(int64_t));
+    const bool flagged = copyResults(tokens_out, log_dev, n_steps * n_seqs * sizeof(int64_t));
     std::vector<int64_t> fed(n_steps);
     for (size_t i = 0; i < n_seqs; ++i) {
         seqLen(seq_ids[i]) += n_steps;
@@ -532,7 +573,9 @@ void Decoder::decodeLoop(const int32_t *seq_ids, size_t n_seqs, const int64_t *f
         }
         recordTokens(seq_ids[i], fed.data(), n_steps);
     }
-    checkKernels();
+    if (flagged) {
+        checkKernels();
+    }
 }
 
 // Error words of the kernels a step ran: the cache's (bad block-table entries, a wait that ran out in an attention

@@ -134,7 +134,11 @@ private:
     size_t &seqLen(int32_t seq);
     void recordTokens(int32_t seq, const int64_t *tokens, size_t n);
     void checkKernels();
+    bool copyResults(void *dst, const void *src, size_t bytes);
+    void freeResults();
 
+    std::byte *_results = nullptr; // page-locked: what a step hands back, and the error words
+    size_t _results_bytes = 0;
     size_t _max_tokens_per_seq = 0;
     std::vector<size_t> _seq_len; // by sequence id; SIZE_MAX = not live
     std::vector<int64_t> _seq_last;  // by sequence id: its newest token, -1 when it has none
