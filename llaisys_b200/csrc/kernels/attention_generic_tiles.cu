@@ -237,11 +237,13 @@ __global__ void __launch_bounds__(kThreads, kRows == 64 ? 2 : 1) attention_gener
             for (int o = kLanes / 2; o > 0; o /= 2) {
                 mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
             }
-            const float m_old = m_s[r], m_new = fmaxf(m_old, mx);
+            // (fmaxf drops NaN: where nothing but NaN and -inf has been seen the maximum is still -inf, and the weight of a NaN score must
+            // come out as NaN; hidden scores are -inf and weigh nothing either way)
+            const float m_old = m_s[r], m_new = fmaxf(m_old, mx), base = m_new != -INFINITY ? m_new : 0.f;
             float sum = 0.f;
 #pragma unroll
             for (int i = 0; i < kEach; ++i) {
-                const float e = m_new != -INFINITY && part + kLanes * i < seen ? expf(s[i] - m_new) : 0.f;
+                const float e = expf(s[i] - base);
                 row[part + kLanes * i] = e;
                 sum += e;
             }
@@ -321,7 +323,7 @@ __global__ void __launch_bounds__(kThreads, kRows == 64 ? 2 : 1) attention_gener
 #pragma unroll
         for (int s = 0; s < kMostSplits; ++s) {
             if (s < splits) {
-                const float w = m[s] == -INFINITY ? 0.f : expf(m[s] - m_all);
+                const float w = m[s] == -INFINITY ? 0.f : expf(m[s] - m_all); // (0 x NaN: a share of NaN scores alone still shows)
                 l_all += l[s] * w;
                 o.x += part[s].x * w;
                 o.y += part[s].y * w;

@@ -128,3 +128,33 @@ def test_values_behind_the_mask_stay_out_nvidia(cuda_device, qlen, bad):
     got = helpers.run_self_attention(q, k, v, 128 ** -0.5, llaisys.DeviceType.NVIDIA, "f32")
     assert torch.isfinite(got[:-1]).all() and not torch.isfinite(got[-1]).any()
     assert helpers.max_abs(got[:-1], attention.self_attention_f64(q[:-1], k[:-1], v[:-1], 128 ** -0.5)) <= 1e-5
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), float("-inf")])
+@pytest.mark.parametrize("qlen,kvlen,d", [(1, 1, 128), (2, 20, 64), (3, 200, 128), (8, 700, 64), (40, 40, 128), (96, 97, 64), (96, 777, 128)])  # tiles of 16 rows, of 64
+def test_scores_that_are_not_finite_show_nvidia(cuda_device, qlen, kvlen, d, bad):
+    """A query row, a key in the middle and the first half of the keys that are not finite: in f32 the rows that see one come out as in
+    float64 (NaN, or without the keys of weight zero) and the others untouched. Tolerance: see test_tiles_over_plain_tensors_nvidia."""
+    g = torch.Generator().manual_seed(qlen * kvlen)
+    q, k, v = (workloads.randn((n, h, d), torch.float32, g) for n, h in ((qlen, 12), (kvlen, 2), (kvlen, 2)))
+    tol = 2 * (d + kvlen) * 2.0 ** -24 * v.abs().max().item()
+    sees = torch.arange(kvlen)[None, :] <= torch.arange(qlen)[:, None] + kvlen - qlen
+    for where in ("q", "middle", "half"):
+        q_bad, k_bad = q.clone(), k.clone()
+        if where == "q":
+            q_bad[qlen // 2, 5, 3] = bad
+            rows = torch.arange(qlen) == qlen // 2
+        else:
+            keys = slice(kvlen // 2, kvlen // 2 + 1) if where == "middle" else slice(0, (kvlen + 1) // 2)
+            k_bad[keys, 1, 3] = bad
+            rows = sees[:, keys].any(1)
+        got = helpers.run_self_attention(q_bad, k_bad, v, d ** -0.5, llaisys.DeviceType.NVIDIA, "f32")
+        want = torch.where(rows[:, None, None], attention.self_attention_f64(q_bad, k_bad, v, d ** -0.5),
+                           attention.self_attention_f64(q, k, v, d ** -0.5))
+        # (rows whose only scores are -inf have no weights at all: 0 by this operator's definition, 0 / 0 in the float64 statement)
+        scores = torch.einsum("qhd,khd->qhk", q_bad.double(), k_bad.double().repeat_interleave(6, dim=1))
+        empty = (scores.masked_fill(~sees[:, None, :], -float("inf")) == -float("inf")).all(2)
+        want[empty] = 0
+        assert torch.equal(torch.isnan(got), torch.isnan(want)), (where, torch.isnan(got).any(2).sum(), torch.isnan(want).any(2).sum())
+        assert helpers.max_abs(got.nan_to_num(0), want.nan_to_num(0)) <= tol, where
