@@ -115,8 +115,8 @@ __global__ void __launch_bounds__(kWarps * 32)
         for (int o = 16; o > 0; o >>= 1) {
             mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         }
-        if (mx == -INFINITY) {
-            continue; // no usable key in this block (warp-uniform)
+        if (!__any_sync(0xffffffffu, s != -INFINITY)) {
+            continue; // no usable key in this block (a NaN score, which fmaxf drops, is one: it has to reach the sums)
         }
         const float m_new = fmaxf(m, mx);
         const float alpha = expf(m - m_new); // m = -inf on the first block gives 0

@@ -132,7 +132,8 @@ def test_values_behind_the_mask_stay_out_nvidia(cuda_device, qlen, bad):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("bad", [float("nan"), float("inf"), float("-inf")])
-@pytest.mark.parametrize("qlen,kvlen,d", [(1, 1, 128), (2, 20, 64), (3, 200, 128), (8, 700, 64), (40, 40, 128), (96, 97, 64), (96, 777, 128)])  # tiles of 16 rows, of 64
+@pytest.mark.parametrize("qlen,kvlen,d", [(1, 1, 128), (2, 20, 64), (3, 200, 128), (8, 700, 64), (40, 40, 128), (96, 97, 64), (96, 777, 128),
+                                          (1, 1, 96), (2, 20, 96), (3, 200, 96)])  # tiles of 16 rows, of 64, one CTA per row
 def test_scores_that_are_not_finite_show_nvidia(cuda_device, qlen, kvlen, d, bad):
     """A query row, a key in the middle and the first half of the keys that are not finite: in f32 the rows that see one come out as in
     float64 (NaN, or without the keys of weight zero) and the others untouched. Tolerance: see test_tiles_over_plain_tensors_nvidia."""
