@@ -141,6 +141,10 @@ LLAISYS_API int llaisysPagedKVFlush(llaisysPagedKV_t kv);
  * The chunked-prefill kernel takes part too: it reads its index arrays, sums the work and sets up its on-chip state
  * before waiting, and touches q, K/V, workspace and outputs only after the kernel directly before it has completed. */
 LLAISYS_API int llaisysPagedKVSetLaunchOverlap(llaisysPagedKV_t kv, int enable);
+/* Polls after which a wait of one part of the chunk attention kernel for another gives up (default 1 << 20, about a second at worst; another
+ * limit is for tests and taken by the bf16 form without window, factor or penalty). A call in which one ran out leaves its
+ * output undefined and is reported by llaisysPagedKVCheck; nothing of it is left running. */
+LLAISYS_API int llaisysPagedKVSetWaitLimit(llaisysPagedKV_t kv, uint32_t polls);
 /* LLAISYS_KERNEL_* of this cache's most recent attention call (-1 for a null handle). */
 LLAISYS_API int llaisysPagedKVLastKernel(llaisysPagedKV_t kv);
 /* Synchronises the cache's stream and reports LLAISYS_E_KERNEL if any kernel since the last

@@ -134,6 +134,10 @@ int llaisysPagedKVSetLaunchOverlap(llaisysPagedKV_t kv, int enable) {
     KV_OR_FAIL(kv);
     return guarded([&] { kv->impl.setLaunchOverlap(enable != 0); });
 }
+int llaisysPagedKVSetWaitLimit(llaisysPagedKV_t kv, uint32_t polls) {
+    KV_OR_FAIL(kv);
+    return guarded([&] { kv->impl.setWaitLimit(polls); });
+}
 int llaisysPagedKVFlush(llaisysPagedKV_t kv) {
     KV_OR_FAIL(kv);
     return guarded([&] { kv->impl.flush(); });

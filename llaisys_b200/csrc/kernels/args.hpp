@@ -46,6 +46,7 @@ struct KVView {
     // overlap the tail of the previous kernel on the stream. Contract for the caller: index arrays and block tables were
     // written before that previous kernel started (K/V rows, q and outputs are only touched after it completed).
     bool overlap_launch = false;
+    uint32_t wait_limit = 1u << 20; // polls before a wait inside the chunk kernels gives up (about a second at worst)
     const void *tma_desc = nullptr;      // box = K and V of a page, 64 dims (decode)
     const void *tma_tile_desc = nullptr; // prefill, two maps of 128 bytes: box = one half-tile, 16 slots x 64 dims (K); box = a
                                          // tile as its two halves, 16 slots x 64 dims x 2 (V)

@@ -30,7 +30,8 @@
 // exponentials (2 x 650) and its MMAs (1024) is what is left above 2048.
 //
 // Synchronisation is mbarriers only (and a named barrier per half around the arrival count). Every wait is bounded: one that runs out sets
-// bit 8 of the error word and the CTA winds down. No cluster launch, no multicast.
+// bit 8 of the error word, its warp stops, and the others stop at their next wait. Whatever way a role ends, it sees its own MMAs or copies
+// done before the CTA gives its tensor memory back and leaves. No cluster launch, no multicast.
 #include "kernels.hpp"
 #include "mma_utils.cuh"
 #include "tcgen05_utils.cuh"
@@ -74,7 +75,8 @@ enum : int {
     kBarO = kBarS + 2,               // [2] MMA (commit) -> softmax: the last product of the fragment is done (a barrier of its own: the next
                                      // fragment's first scores may be there before every thread has seen it)
     kBarTurn = kBarO + 2,            // [2] issuer of the other half -> issuer of this half: its batch is issued, the next one is yours
-    kBarP = kBarTurn + 2,            // [2][2] softmax (128) -> MMA: this part of P is in tensor memory (and the accumulator rescaled)
+    kBarDrain = kBarTurn + 2,        // [2] MMA (commit) -> the issuer itself: everything it issued has finished
+    kBarP = kBarDrain + 2,           // [2][2] softmax (128) -> MMA: this part of P is in tensor memory (and the accumulator rescaled)
     kBarQ = kBarP + 4,               // [2] softmax (128) -> MMA: the next fragment's Q rows are in shared memory
     kNumBars = kBarQ + 2
 };
@@ -102,6 +104,7 @@ struct ChunkParams {
     long long out_stride; // elements between rows of out
     const float *row_scale;
     const float *fade_a, *fade_b; // fading instantiation: fade_a[h] log2(1 + fade_b[h] (distance)) is taken off the scores in the log2 domain
+    uint32_t wait_limit;          // polls before a wait gives up, where not kMbarWaitLimit
     int32_t out_wide;             // out is 32-byte aligned: rows are stored 32 bytes (a whole sector) per instruction
 };
 
@@ -287,7 +290,7 @@ enum Form {
     kFading,   // the same with a distance penalty
 };
 
-template <bool kBf16, int kForm>
+template <bool kBf16, int kForm, bool kShortWaits>
 __global__ void __launch_bounds__(kThreads, 1)
     paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap tmap_v, ChunkParams p) {
     constexpr bool kWin = kForm != kPlain, kFade = kForm == kFading;
@@ -427,9 +430,20 @@ __global__ void __launch_bounds__(kThreads, 1)
     const uint32_t tmem_base = *s_tmem_base;
 
     auto bar = [&](int which) { return bars_u32 + uint32_t(which) * 8; };
-    auto give_up = [&]() {
-        *s_abort = 1;
-        atomicOr(p.error_flag, kErrTimeout);
+    // False when the wait ran out here or somewhere else in the CTA (lanes may disagree on that); raises the flag that ends the others.
+    auto wait = [&](int which, uint32_t parity) {
+        const bool ok = wait_or_abort(bar(which), parity & 1u, s_abort, kShortWaits ? p.wait_limit : kMbarWaitLimit);
+        if (!ok) {
+            *s_abort = 1;
+        }
+        return ok;
+    };
+    // For what is on its way in any case: not cut short by another warp's failure.
+    auto drain = [&](int which, uint32_t parity) {
+        if (!mbar_wait_bounded(bar(which), parity & 1u, kMbarWaitLimit)) {
+            *s_abort = 1;
+        }
+        __syncwarp();
     };
     // A warp's place on the line waits in shared memory while its blocks run: a register that is spilled there is fetched from L2 (the
     // operands leave no L1), and a dozen such loads per block cost as much as the block.
@@ -486,10 +500,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                     const int row = int((p.page0 + page) * 2); // K of the page; V is the next index
 #pragma unroll
                     for (int is_v = 0; is_v < 2; ++is_v) {
-                        if (turn > 0 && !wait_or_abort(bar(kBarEmpty + stage), (turn - 1) & 1u, s_abort)) {
-                            if (lane == 0) {
-                                give_up();
-                            }
+                        if (turn > 0 && !__all_sync(0xffffffffu, wait(kBarEmpty + stage, turn - 1))) {
                             alive = false;
                             break;
                         }
@@ -525,23 +536,23 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
                 pos += n;
             }
+            for (int load = max(int(turn) * kStages + stage - kStages, 0); load < int(turn) * kStages + stage; ++load) {
+                drain(kBarFull + load % kStages, uint32_t(load / kStages));
+            }
         } else if (warp <= kMmaWarp + 1) {
             // ================================ MMA issuers, one warp per half ========================================
             // tcgen05.mma is accepted at the pace of the tensor pipe, a few instructions ahead: with one warp for both halves the pipe stood idle
             // through every wait, commit and loop step between batches (2100 of a block's 4200 clocks). With two, one half's batch runs under the
-            // other's waits. The whole warp walks the blocks and one lane issues: descriptors then come from uniform registers. A wait that runs out
-            // raises the abort flag and goes on: later waits give up soon, nothing here leaves the CTA.
+            // other's waits. The whole warp walks the blocks and one lane issues: descriptors then come from uniform registers.
+            // A lane whose wait ran out issues nothing any more and skips its later waits, but walks on: the warp stays together without a vote per
+            // wait (with one, a prompt of 8192 took 587 instead of 558 us).
             const int h = __shfl_sync(0xffffffffu, warp, 0) - kMmaWarp;
             constexpr uint32_t idesc_qk = make_idesc(kBf16, false, kHalf, kKeys), idesc_pv = make_idesc(kBf16, true, kHalf, kD);
             const uint32_t tmem_s = __shfl_sync(0xffffffffu, tmem_base, 0) + kColS + h * kKeys, tmem_o = __shfl_sync(0xffffffffu, tmem_base, 0) + kColO + h * kD;
             const uint64_t q_desc = smem_desc_sw128(base_u32 + h * kQBytes, 0, 1024), k_desc = smem_desc_sw128(ring_u32, 0, 1024),
                            v_desc = smem_desc_sw128(ring_u32, 2048, 1024);
             const bool leader = elect_one();
-            auto wait = [&](int which, uint32_t parity) {
-                if (!wait_or_abort(bar(which), parity & 1u, s_abort) && lane == 0) {
-                    give_up();
-                }
-            };
+            bool ok = true;
             int stage = 0;
             uint32_t turn = 0, p_turn = 0, q_turn = 0, my_turn = 0;
             // Where both halves have rows their batches alternate: left to themselves they fall into step, both softmaxes at once (and short of
@@ -549,20 +560,20 @@ __global__ void __launch_bounds__(kThreads, 1)
             bool two = false;
             auto take_turn = [&]() {
                 if (two && (h == 1 || my_turn > 0)) {
-                    wait(kBarTurn + h, h == 1 ? my_turn : my_turn - 1);
+                    ok = ok && wait(kBarTurn + h, h == 1 ? my_turn : my_turn - 1);
                 }
                 my_turn += two ? 1u : 0u;
             };
             auto take_stage = [&]() { // the next stage of the ring, once it has landed
                 const int s = stage;
-                wait(kBarFull + s, turn);
+                ok = ok && wait(kBarFull + s, turn);
                 stage = s + 1 == kStages ? 0 : s + 1;
                 turn += s + 1 == kStages ? 1u : 0u;
                 return s;
             };
             auto issue_qk = [&](int s) {
                 const uint64_t k = k_desc + uint64_t(s * (kStageBytes >> 4));
-                if (leader) {
+                if (leader && ok) {
 #pragma unroll
                     for (int ks = 0; ks < kD / 16; ++ks) {
                         umma_f16(tmem_s, q_desc + uint64_t(((ks >> 2) * kQPiece + (ks & 3) * 32) >> 4), k + uint64_t(((ks >> 2) * kPieceBytes + (ks & 3) * 32) >> 4),
@@ -571,7 +582,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
             };
             auto commit = [&](int which) {
-                if (leader) {
+                if (leader && ok) {
                     umma_commit(bar(which));
                     if (two) {
                         mbar_arrive(bar(kBarTurn + 1 - h));
@@ -594,14 +605,14 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (h == 1 && !two) { // no rows: see the stages pass (every phase in order) and free them
                     for (int i = 0; i < 2 * n; ++i) {
                         const int s = take_stage();
-                        if (lane == 0) {
+                        if (ok && lane == 0) {
                             mbar_arrive(bar(kBarEmpty + s));
                         }
                     }
                     continue;
                 }
                 const int k0 = take_stage();
-                wait(kBarQ + h, q_turn++);
+                ok = ok && wait(kBarQ + h, q_turn++);
                 take_turn();
                 issue_qk(k0);
                 commit(kBarS + h);
@@ -611,12 +622,12 @@ __global__ void __launch_bounds__(kThreads, 1)
                     const uint64_t v = v_desc + uint64_t(v_at * (kStageBytes >> 4));
 #pragma unroll
                     for (int part = 0; part < 2; ++part) {
-                        wait(kBarP + h * 2 + part, p_turn);
+                        ok = ok && wait(kBarP + h * 2 + part, p_turn);
                         if (part == 0) {
                             take_turn();
                         }
                         tc_fence_after();
-                        if (leader) {
+                        if (leader && ok) {
 #pragma unroll
                             for (int k4 = 0; k4 < kPagesPerBlock / 2; ++k4) {
                                 // B = 16 keys (one page) x 128 dims of V, MN-major: 8-key groups 1 KiB apart, the page's two 64-dim halves 2 KiB
@@ -633,6 +644,11 @@ __global__ void __launch_bounds__(kThreads, 1)
                     commit((more ? kBarS : kBarO) + h);
                 }
             }
+            if (leader) {
+                umma_commit(bar(kBarDrain + h));
+            }
+            __syncwarp();
+            drain(kBarDrain + h, 0);
         }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(kSoftmaxRegs));
@@ -666,9 +682,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             fence_proxy_async_smem(); // read by the async proxy
             mbar_arrive(bar(kBarQ + h));
         };
-        // A thread whose wait ran out stops computing but keeps walking the fragments, so that the named barrier and the arrival counts
-        // below see all 128 threads every time.
-        bool dead = false;
+        // A lane whose wait ran out goes on with what it finds, so that the warp stays together (without a vote per block, which took 2 % of
+        // a prompt, and with one flag less in the block loop) and the named barrier and the arrival counts below see all 128 threads every
+        // time. Nothing of a fragment is stored once the CTA has given up.
         uint32_t s_turn = 0, o_turn = 0;
         // stages that this half has seen read: K of block b is load 2 b of the CTA, V load 2 b + 1
         int done = 0; // blocks of earlier fragments
@@ -676,10 +692,6 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (row == 0) {
                 mbar_arrive(bar(kBarEmpty + load % kStages));
             }
-        };
-        auto wait_s = [&]() {
-            dead = dead || !wait_or_abort(bar(kBarS + h), s_turn++ & 1u, s_abort);
-            tc_fence_after();
         };
         int pos = piece_begin;
         bool more = false;
@@ -690,7 +702,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 pos += f.b1 - f.b0;
                 done += f.b1 - f.b0;
             }
-            if (more && !dead) {
+            if (more) {
                 load_q(f, w.g);
             }
             keep_place(w, f);
@@ -706,10 +718,8 @@ __global__ void __launch_bounds__(kThreads, 1)
             float m_used = -INFINITY, l = 0.f;
             const float fade_a = kFade ? p.fade_a[head] : 0.f, fade_b = kFade ? p.fade_b[head] : 0.f;
             for (int i = 0; i < n; ++i) {
-                wait_s();
-                if (dead) {
-                    break;
-                }
+                wait(kBarS + h, s_turn++);
+                tc_fence_after();
                 free_stage(2 * (done + i));
                 if (i >= 1) {
                     free_stage(2 * (done + i) - 1);
@@ -843,11 +853,10 @@ __global__ void __launch_bounds__(kThreads, 1)
             done += n;
             move_on();
             // ---- epilogue of the fragment ---------------------------------------------------------------------------
-            dead = dead || !wait_or_abort(bar(kBarO + h), o_turn++ & 1u, s_abort);
+            wait(kBarO + h, o_turn++);
             tc_fence_after();
-            if (!dead) {
-                free_stage(last_load);
-            }
+            free_stage(last_load);
+            const bool dead = __any_sync(0xffffffffu, *s_abort != 0) != 0;
             const bool whole = f.b0 == 0 && f.b1 == f.tile_nblk;
             bool store_rows = whole;
             float w_own = 1.f, l_all = l, m_all = m_used;
@@ -973,15 +982,15 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
             tc_fence_before(); // the O reads above come before the next fragment's P arrival in program order
         }
-        if (dead && lane == 0) {
-            give_up();
-        }
     }
 
     // ---- teardown: everyone is done with TMEM before the allocating warp frees it ----------------------------------
     __syncwarp();
     tc_fence_before();
     __syncthreads();
+    if (tid == 0 && *s_abort != 0) {
+        atomicOr(p.error_flag, kErrTimeout);
+    }
     if (warp == kMmaWarp) {
         tc_fence_after();
         tmem_dealloc(tmem_base, kTmemCols);
@@ -1024,13 +1033,13 @@ int chunk_slots() {
     return n;
 }
 
-template <bool kBf16, int kForm>
+template <bool kBf16, int kForm, bool kShortWaits = false>
 void launch(cudaStream_t s, const CUtensorMap &tmap, const CUtensorMap &tmap_v, const ChunkParams &p, int grid, bool overlap) {
     static std::once_flag once[64];
     int dev = 0;
     LLAISYS_CUDA_CHECK(cudaGetDevice(&dev));
     std::call_once(once[dev & 63], [] {
-        LLAISYS_CUDA_CHECK(cudaFuncSetAttribute(paged_prefill_tc_kernel<kBf16, kForm>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemBytes)));
+        LLAISYS_CUDA_CHECK(cudaFuncSetAttribute(paged_prefill_tc_kernel<kBf16, kForm, kShortWaits>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemBytes)));
     });
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(unsigned(grid));
@@ -1042,7 +1051,7 @@ void launch(cudaStream_t s, const CUtensorMap &tmap, const CUtensorMap &tmap_v, 
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = overlap ? 1 : 0;
-    LLAISYS_CUDA_CHECK(cudaLaunchKernelEx(&cfg, paged_prefill_tc_kernel<kBf16, kForm>, tmap, tmap_v, p));
+    LLAISYS_CUDA_CHECK(cudaLaunchKernelEx(&cfg, paged_prefill_tc_kernel<kBf16, kForm, kShortWaits>, tmap, tmap_v, p));
 }
 
 } // namespace
@@ -1177,6 +1186,7 @@ int attention_prefill_tc(stream_t stream, llaisysDataType_t dtype, const KVView 
     p.out = out.out;
     p.scale_log2 = scale * 1.4426950408889634f;
     p.error_flag = error_flag;
+    p.wait_limit = kv.wait_limit;
     // the workspace of the split tiles: the halves of two fragments per CTA, and an arrival counter per half
     const int grid = chunk_slots();
     if (scratch.partials == nullptr || scratch.counters == nullptr ||
@@ -1210,7 +1220,9 @@ int attention_prefill_tc(stream_t stream, llaisysDataType_t dtype, const KVView 
         constexpr int kForm = decltype(form)::value;
         bf16 ? launch<true, kForm>(s, tmap, tmap_v, p, grid, kv.overlap_launch) : launch<false, kForm>(s, tmap, tmap_v, p, grid, kv.overlap_launch);
     };
-    if (fading) {
+    if (p.wait_limit != kMbarWaitLimit && bf16 && !windowed) { // (a limit that tests set: by value it costs every block's waits 2 %)
+        launch<true, kPlain, true>(s, tmap, tmap_v, p, grid, kv.overlap_launch);
+    } else if (fading) {
         run(std::integral_constant<int, kFading>{});
     } else if (windowed) {
         run(std::integral_constant<int, kWindowed>{});

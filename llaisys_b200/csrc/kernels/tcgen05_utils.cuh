@@ -153,8 +153,8 @@ __device__ __forceinline__ bool elect_one() { // one lane of a converged warp
     return leader != 0;
 }
 
-__device__ __forceinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
-    for (uint32_t i = 0; i < kMbarWaitLimit; ++i) {
+__device__ __forceinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, volatile int *abort_flag, uint32_t limit = kMbarWaitLimit) {
+    for (uint32_t i = 0; i < limit; ++i) {
         if (mbar_try_wait(bar, parity)) {
             return true;
         }

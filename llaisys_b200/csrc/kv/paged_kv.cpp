@@ -534,6 +534,7 @@ kernels::KVView PagedKV::view(size_t layer) const {
         v.v_token_stride = int64_t(l.v_row);
     }
     v.overlap_launch = _overlap;
+    v.wait_limit = _wait_limit;
     if (l.has_tma) {
         v.tma_tile_desc = l.tma_tile_desc;
         v.tma_desc = l.tma_desc;

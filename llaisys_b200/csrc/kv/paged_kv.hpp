@@ -90,6 +90,7 @@ public:
     size_t layerBytes() const { return _layers[0].bytes; } // of layer 0; all layers' when they have one shape
     const int32_t *blockTableData() const { return reinterpret_cast<const int32_t *>(_table_dev->memory()); }
     void setLaunchOverlap(bool enable) { _overlap = enable; }
+    void setWaitLimit(uint32_t polls) { _wait_limit = polls; }
     // LLAISYS_KERNEL_* id of the kernel that served this cache's most recent attention call
     int lastKernel() const { return _last_kernel; }
     void flush(); // queue uploads of the table rows that changed since the last flush
@@ -229,6 +230,7 @@ private:
     uint32_t _seen_epoch = 0;
     const void *_host_stage_alias = nullptr; // device-side address of _host_stage (mapped page-locked memory)
 
+    uint32_t _wait_limit = kernels::KVView().wait_limit;
     bool _overlap = false; // launch append / decode with programmatic stream serialisation
     int _last_kernel = 0;
 };

@@ -355,6 +355,7 @@ PROTOTYPES: dict[str, tuple] = {
     "llaisysPagedKVBlockTableData": (c_void_p, [_KV]),
     "llaisysPagedKVFlush": (c_int, [_KV]),
     "llaisysPagedKVSetLaunchOverlap": (c_int, [_KV, c_int]),
+    "llaisysPagedKVSetWaitLimit": (c_int, [_KV, ctypes.c_uint32]),
     "llaisysPagedKVCheck": (c_int, [_KV]),
     "llaisysPagedKVAppend": (c_int, [_KV, c_size_t, c_void_p, c_void_p, _I32P, _I32P, c_size_t]),
     "llaisysPagedKVGather": (c_int, [_KV, c_size_t, c_int32, c_size_t, c_void_p, c_void_p]),

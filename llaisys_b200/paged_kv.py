@@ -171,6 +171,10 @@ class PagedKVCache:
         """Opt in to programmatic dependent launch of append / decode (see llaisysPagedKVSetLaunchOverlap)."""
         _check(LIB_LLAISYS.llaisysPagedKVSetLaunchOverlap(self._kv, 1 if enable else 0))
 
+    def set_wait_limit(self, polls: int) -> None:
+        """Polls after which a wait inside chunk attention gives up and check() reports it (see llaisysPagedKVSetWaitLimit)."""
+        _check(LIB_LLAISYS.llaisysPagedKVSetWaitLimit(self._kv, polls))
+
     def last_kernel(self) -> "Kernel":
         """Which kernel served this cache's most recent attention call."""
         return Kernel(LIB_LLAISYS.llaisysPagedKVLastKernel(self._kv))

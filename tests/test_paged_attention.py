@@ -815,3 +815,41 @@ def test_prefill_rows_packed_over_the_heads_of_a_group_nvidia(cuda_device, dname
             s = torch.einsum("thd,jhd->htj", q[starts[i]:starts[i + 1]].double(), k) * scale
             want = torch.einsum("htj,jhd->thd", s.masked_fill(hidden, -np.inf).softmax(-1), v)
             assert helpers.max_abs(out[starts[i]:starts[i + 1]], want) <= helpers.MAX_ABS[dname] * max(1.0, want.abs().max().item() / 4), (i, scale)
+
+
+@pytest.mark.gpu
+def test_chunk_waits_that_run_out_are_reported_nvidia(cuda_device):
+    """With a limit of a few polls the waits inside a healthy pipeline run out, from the first on or somewhere in the middle: the call ends,
+    is reported, and the next one, with the limit as it was, gives the bits of the one before."""
+    nh, nkvh, d = 12, 2, 128
+    q_lens, before = [700, 1, 40, 300], [1000, 0, 5, 4000]
+    kv_lens = [q + b for q, b in zip(q_lens, before)]
+    g = torch.Generator().manual_seed(5)
+    ks, vs = ([workloads.randn((n, nkvh, d), torch.bfloat16, g) for n in kv_lens] for _ in range(2))
+    q = workloads.randn((sum(q_lens), nh, d), torch.bfloat16, g).cuda()
+    counts = [-(-n // 16) for n in kv_lens]
+    ends = np.cumsum(counts)
+    cache, seqs = helpers.build_cache(NVIDIA, "bf16", [list(range(e - n, e)) for e, n in zip(ends, counts)], num_pages=int(ends[-1]), nkvh=nkvh, d=d)
+    helpers.append_all(cache, 0, seqs, ks, vs, NVIDIA)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")  # noqa: E731
+    ids, starts, lens = i32(seqs), i32([0, *np.cumsum(q_lens).tolist()]), i32(kv_lens)
+    out = torch.empty_like(q)
+
+    def attend():
+        out.fill_(float("nan"))
+        torch.cuda.synchronize()
+        cache.prefill_dev(0, out, q, ids, starts, lens, len(seqs), sum(q_lens), max(q_lens), max(kv_lens), nh, d ** -0.5, llaisys.context_stream())
+        cache.check()
+        return out.clone()
+
+    first = attend()
+    assert torch.isfinite(first).all()
+    for polls in (0, 1, 2, 4, 8, 16, 64, 0):
+        cache.set_wait_limit(polls)
+        try:
+            attend()
+            assert polls > 0
+        except LlaisysError as e:
+            assert e.status == Status.KERNEL
+        cache.set_wait_limit(1 << 20)
+        assert torch.equal(attend(), first), polls
