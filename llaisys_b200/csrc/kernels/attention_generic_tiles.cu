@@ -391,8 +391,12 @@ bool attention_generic_tiles(stream_t stream, llaisysDataType_t dtype, const KVV
                        out.row_stride == 0 && kv.vDim() == kv.d && (kv.d == 64 || kv.d == 128) && kv.head_stride == kv.d &&
                        kv.token_stride == int64_t(kv.nkvh) * kv.d && kv.page_stride == kv.page_size * kv.token_stride;
     auto aligned = [](const void *ptr) { return reinterpret_cast<uintptr_t>(ptr) % 16 == 0; }; // q, K and V come in pieces of 16 bytes
+    // Up to 16 keys a tile is mostly padding and the cluster's start-up is the call. One CTA per (row, head) takes 6.5, 8.7 and 10.7 us for 4, 8
+    // and 16 keys with heads of 64, 8.7, 10.7 and 12.8 with heads of 128; tiles take 10.7 and 12.8 to 14.8 up to 32 keys, where the other
+    // kernel is at 15 and 18.
+    constexpr int kFewKeys = 16;
     if (!plain || !aligned(q) || !aligned(kv.k_base) || !aligned(kv.v_base) || kv.nkvh > 65535 || batch.total_q != batch.const_q_len ||
-        batch.const_kv_len < batch.const_q_len || int64_t(batch.total_q) * (batch.nh / kv.nkvh) > (int64_t(1) << 27)) {
+        batch.const_kv_len < batch.const_q_len || batch.const_kv_len <= kFewKeys || int64_t(batch.total_q) * (batch.nh / kv.nkvh) > (int64_t(1) << 27)) {
         return false;
     }
     const TileParams p{q, kv.k_base, kv.v_base, out.out, batch.total_q, batch.const_kv_len, batch.nh, kv.nkvh, scale};

@@ -103,7 +103,7 @@ def test_multi_token_queries_over_plain_tensors_nvidia(cuda_device, qlen, kvlen,
 @pytest.mark.gpu
 @pytest.mark.parametrize("dname", ["f32", "f16", "bf16"])
 @pytest.mark.parametrize("qlen,kvlen,nh,nkvh,d", [
-    (1, 1, 12, 2, 64), (1, 129, 12, 2, 128), (2, 128, 12, 2, 128), (15, 127, 5, 1, 128), (15, 900, 18, 2, 128),  # tiles of 16 rows
+    (1, 1, 12, 2, 64), (5, 16, 12, 2, 64), (5, 17, 12, 2, 64), (1, 129, 12, 2, 128), (2, 128, 12, 2, 128), (15, 127, 5, 1, 128), (15, 900, 18, 2, 128),  # tiles of 16 rows
     (65, 65, 32, 8, 64), (86, 300, 12, 2, 64), (96, 777, 12, 2, 128), (300, 301, 12, 2, 64), (257, 513, 33, 3, 128)])  # tiles of 64 rows
 def test_tiles_over_plain_tensors_nvidia(cuda_device, qlen, kvlen, nh, nkvh, d, dname):
     """Calls that neither 16-bit kernel takes: tiles that end inside the rows, key blocks that end inside a split, groups that do not
