@@ -8,7 +8,7 @@
 // and a TILE is (sequence, 256 packed rows, kv head). Tiles of 128 queries of one head, as before, filled a chunk of 20 tokens to a sixth
 // and fetched K and V once per head. A tile visits its visible keys 128 at a time (a BLOCK: 8 pages). All blocks of all tiles, in the order
 // (sequence, row block, kv head, key block), form one line that is cut into equal pieces, one per SM, so that every SM gets the same number
-// of blocks whatever the mix of lengths. A piece covers the end of one tile, whole tiles, and the beginning of another; each such FRAGMENT
+// of blocks whatever the mix of lengths; where tiles are short, whole tiles are dealt out instead. A piece covers the end of one tile, whole tiles, and the beginning of another; each such FRAGMENT
 // runs like a tile. A fragment that is its whole tile normalises and stores its rows; otherwise it stores the accumulator and the rows' (max,
 // sum) into a slot of a workspace and counts itself in, and the fragment that arrives last merges the others with what it holds, in the
 // order of the CTAs and not of arrival. Nobody waits for another CTA.
@@ -30,8 +30,8 @@
 // exponentials (2 x 650) and its MMAs (1024) is what is left above 2048.
 //
 // Synchronisation is mbarriers only (and a named barrier per half around the arrival count). Every wait is bounded: one that runs out sets
-// bit 8 of the error word, its warp stops, and the others stop at their next wait. Whatever way a role ends, it sees its own MMAs or copies
-// done before the CTA gives its tensor memory back and leaves. No cluster launch, no multicast.
+// bit 8 of the error word, its lane hands nothing on any more, and the others give up at their next wait. Whatever way a role ends, it sees
+// its own MMAs or copies done before the CTA gives its tensor memory back and leaves. No cluster launch, no multicast.
 #include "kernels.hpp"
 #include "mma_utils.cuh"
 #include "tcgen05_utils.cuh"
@@ -55,7 +55,8 @@ constexpr int kSoftmaxThreads = 128, kProducerWarp = 8, kMmaWarp = 9, kThreads =
 // Registers a thread: 384 x 168 at launch, then 256 softmax threads take 224 and the 128 of the other four warps (one of them idle) keep 56.
 constexpr int kSoftmaxRegs = 224, kOtherRegs = 56;
 static_assert(256 * kSoftmaxRegs + 128 * kOtherRegs <= kThreads * 168, "no more than the CTA was launched with");
-constexpr int kPlaceInts = 24; // words of shared memory in which a warp keeps its place on the line
+constexpr int kSchedInts = 44; // sums, maxima and tiles of twelve warps; start of the piece, arrivals, the piece
+constexpr int kPlaceInts = 25; // words of shared memory in which a warp keeps its place on the line
 constexpr int kTmemCols = 512, kColS = 0, kColO = 2 * kKeys; // scores of half h at kColS + 128 h, accumulators at kColO + 128 h
 constexpr int kErrTimeout = 8;
 constexpr float kRescaleThreshold = 8.f; // log2 units
@@ -64,6 +65,7 @@ constexpr int kPartialFloats = kHalf * kD + 2 * kHalf;
 // Merging a partial costs its reader about as much as kMergeCostBlocks blocks; shorter pieces than sqrt(kMergeCostBlocks * longest tile)
 // would spend more on merging than they save.
 constexpr float kMergeCostBlocks = 1.5f;
+constexpr int kMergeCost = 2; // (for a tile in two or three pieces)
 // What a tile costs besides its blocks (loading Q, draining the pipeline, storing its rows: about 11500 clocks), in units of a block's time.
 constexpr int kTileCost = 4;
 
@@ -80,7 +82,7 @@ enum : int {
     kBarQ = kBarP + 4,               // [2] softmax (128) -> MMA: the next fragment's Q rows are in shared memory
     kNumBars = kBarQ + 2
 };
-constexpr size_t kSmemBytes = 1024 + 2 * size_t(kQBytes) + kStages * size_t(kStageBytes) + kNumBars * 8 + 8 + 32 * sizeof(int) +
+constexpr size_t kSmemBytes = 1024 + 2 * size_t(kQBytes) + kStages * size_t(kStageBytes) + kNumBars * 8 + 8 + kSchedInts * sizeof(int) +
                               kThreads / 32 * kPlaceInts * sizeof(int);
 static_assert(kSmemBytes <= 227 * 1024, "shared memory of an SM");
 
@@ -163,10 +165,13 @@ __device__ __forceinline__ int floor_sum(int n, int m, int b) {
     }
     return sum;
 }
-// units of the line in front of row block qb of a sequence (qb < n_qb), per kv head: the tiles' blocks in closed form -- tile i ends at key
-// floor((256 i + 255) / group) + 1 + off, so it has floor((2 i + B) / group) blocks, and its gap is such a term too -- and kTileCost each
-__device__ __forceinline__ int units_before(const SeqGeom &g, int qb) {
+// Units of the line in front of row block qb of a sequence (qb < n_qb), per kv head. Whole tiles: one each. Else the tiles' blocks in closed
+// form -- tile i ends at key floor((256 i + 255) / group) + 1 + off, so it has floor((2 i + B) / group) blocks, and its gap is such a term too -- and kTileCost each
+__device__ __forceinline__ int units_before(const SeqGeom &g, int qb, bool whole) {
     static_assert(kRows == 2 * kKeys, "row blocks advance two key blocks over the group's heads");
+    if (whole) {
+        return qb;
+    }
     int units = qb * kTileCost + floor_sum(qb, g.group, (kRows - 1 + g.group * (g.off + kKeys)) >> 7);
     if (g.window > 0) {
         const int c = g.group * (g.off - g.window + 1 - g.kept_blocks * kKeys), q0 = c >= 0 ? 0 : (-c + kRows - 1) / kRows;
@@ -177,8 +182,11 @@ __device__ __forceinline__ int units_before(const SeqGeom &g, int qb) {
     return units;
 }
 // units of a whole sequence
-__device__ __forceinline__ int seq_units(const ChunkParams &p, const SeqGeom &g) {
-    return g.n_qb == 0 ? 0 : (units_before(g, g.n_qb - 1) + tile_blocks(g, g.n_qb - 1) + kTileCost) * p.nkvh;
+__device__ __forceinline__ int seq_units(const ChunkParams &p, const SeqGeom &g, bool whole) {
+    if (whole || g.n_qb == 0) {
+        return g.n_qb * p.nkvh;
+    }
+    return (units_before(g, g.n_qb - 1, false) + tile_blocks(g, g.n_qb - 1) + kTileCost) * p.nkvh;
 }
 
 // Position on the line: every role of the CTA walks the same fragments with one of these.
@@ -188,6 +196,7 @@ struct Walker {
     int n_units;   // its units (all kv heads)
     SeqGeom g;
     int qb, qb_begin; // the row block of the last position asked for, and its first unit inside the sequence (positions only move forward)
+    bool whole;       // a unit is a whole tile
 };
 
 struct Fragment {
@@ -197,10 +206,12 @@ struct Fragment {
     int tile_nblk;  // blocks of the whole tile
     int tile_begin; // index on the line of the tile's block 0
     int rows;       // live rows of the tile
+    int units;      // from its first unit to the position behind it
 };
 struct Place {
     Walker w;
     Fragment f;
+    int pos; // on the line, behind the fragment
 };
 static_assert(sizeof(Place) <= kPlaceInts * sizeof(int), "a warp's words");
 
@@ -212,21 +223,22 @@ __device__ __forceinline__ bool locate(const ChunkParams &p, Walker &w, int &pos
             w.seq_begin += w.n_units;
             ++w.a;
             w.g = seq_geom(p, w.a);
-            w.n_units = seq_units(p, w.g);
+            w.n_units = seq_units(p, w.g, w.whole);
             w.qb = w.qb_begin = 0;
         }
-        int x = pos - w.seq_begin - w.qb_begin, nb = tile_blocks(w.g, w.qb);
-        while (x >= (nb + kTileCost) * p.nkvh && w.qb + 1 < w.g.n_qb) {
-            x -= (nb + kTileCost) * p.nkvh;
-            w.qb_begin += (nb + kTileCost) * p.nkvh;
+        int x = pos - w.seq_begin - w.qb_begin, nb = tile_blocks(w.g, w.qb), span = w.whole ? 1 : nb + kTileCost;
+        while (x >= span * p.nkvh && w.qb + 1 < w.g.n_qb) {
+            x -= span * p.nkvh;
+            w.qb_begin += span * p.nkvh;
             nb = tile_blocks(w.g, ++w.qb);
+            span = w.whole ? 1 : nb + kTileCost;
         }
-        const int kvh = min(x / (nb + kTileCost), p.nkvh - 1), b0 = x - kvh * (nb + kTileCost);
-        if (b0 >= nb + kTileCost) {
+        const int kvh = min(x / span, p.nkvh - 1), b0 = x - kvh * span;
+        if (b0 >= span) {
             return false; // (past the end of the line: no caller asks)
         }
         if (b0 >= nb) { // behind the tile's last block: on to the next tile
-            pos += nb + kTileCost - b0;
+            pos += span - b0;
             continue;
         }
         f.a = w.a;
@@ -235,7 +247,8 @@ __device__ __forceinline__ bool locate(const ChunkParams &p, Walker &w, int &pos
         f.b0 = b0;
         f.tile_nblk = nb;
         f.gap = tile_gap(w.g, w.qb);
-        f.b1 = min(nb, b0 + (piece_end - pos));
+        f.b1 = w.whole ? nb : min(nb, b0 + (piece_end - pos));
+        f.units = w.whole ? 1 : f.b1 - b0;
         f.tile_begin = pos - b0;
         f.rows = min(kRows, w.g.q_len * w.g.group - w.qb * kRows);
         return true;
@@ -303,19 +316,20 @@ __global__ void __launch_bounds__(kThreads, 1)
     const uint32_t bars_u32 = smem_u32(bars);
     uint32_t *s_tmem_base = reinterpret_cast<uint32_t *>(bars + kNumBars);
     volatile int *s_abort = reinterpret_cast<volatile int *>(s_tmem_base + 1);
-    int *s_sched = reinterpret_cast<int *>(s_tmem_base + 2); // [32]: sums and maxima of the warps, start of the piece, arrival order
+    int *s_sched = reinterpret_cast<int *>(s_tmem_base + 2); // [kSchedInts]
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     constexpr int kWarps = kThreads / 32;
 
     // ---- this CTA's piece of the line ----------------------------------------------------------------------------
     // (every CTA sums the sequences' units itself: a few loads per sequence, no launch in front of this one)
-    int line_units = 0, longest_tile = 0;
+    int line_units = 0, longest_tile = 0, tiles = 0;
     {
-        int mine = 0, mine_max = 0;
+        int mine = 0, mine_max = 0, mine_tiles = 0;
         for (int a = tid; a < p.n_seqs; a += kThreads) {
             const SeqGeom g = seq_geom(p, a);
-            mine += seq_units(p, g);
+            mine += seq_units(p, g, false);
+            mine_tiles += seq_units(p, g, true);
             // (with a window: what a tile can reach, it only sizes the pieces)
             const int reach = g.window > 0 ? (g.window + kRows / g.group + kKeys) / kKeys + 1 + g.kept_blocks : 1 << 30;
             mine_max = max(mine_max, g.n_qb > 0 ? min((g.kv_len + kKeys - 1) / kKeys, reach) : 0);
@@ -324,33 +338,50 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int d = 16; d > 0; d >>= 1) {
             mine += __shfl_xor_sync(0xffffffffu, mine, d);
             mine_max = max(mine_max, __shfl_xor_sync(0xffffffffu, mine_max, d));
+            mine_tiles += __shfl_xor_sync(0xffffffffu, mine_tiles, d);
         }
         if (lane == 0) {
             s_sched[warp] = mine;
             s_sched[kWarps + warp] = mine_max;
+            s_sched[2 * kWarps + warp] = mine_tiles;
         }
         __syncthreads();
         for (int w = 0; w < kWarps; ++w) {
             line_units += s_sched[w];
             longest_tile = max(longest_tile, s_sched[kWarps + w]);
+            tiles += s_sched[2 * kWarps + w];
         }
     }
     const int n_slots = int(gridDim.x);
     const int min_piece = int(ceilf(sqrtf(kMergeCostBlocks * float(longest_tile))));
-    const int piece = max((line_units + n_slots - 1) / n_slots, max(min_piece, kTileCost + 1)); // units per CTA
+    int piece = max((line_units + n_slots - 1) / n_slots, max(min_piece, kTileCost + 1)); // units per CTA
+    // A cut costs its second CTA what a tile costs, and the merge: where no CTA has more to do with whole tiles alone, there are no cuts.
+    // (24 chunks of 100 tokens behind 200, 12 / 2 heads, are 144 tiles of three blocks: cut into equal pieces nearly every CTA had parts of two
+    // tiles, 35 us a layer; whole 22.)
+    const int tiles_each = (tiles + n_slots - 1) / n_slots;
+    const bool whole = (long long)tiles_each * (longest_tile + kTileCost) <= piece + kTileCost + kMergeCost;
+    if (whole) {
+        piece = tiles_each;
+        line_units = tiles;
+    }
     const int slot = int(blockIdx.x);
     const int piece_begin = slot * piece;
     if (piece_begin >= line_units) {
         return; // uniform over the CTA, before any mbarrier or TMEM allocation
     }
     const int piece_end = min(line_units, piece_begin + piece);
+    volatile int *s_line = s_sched + 3 * kWarps + 4; // units per piece, end of this one (kept there for the same reason as a warp's place)
+    if (tid == 0) {
+        s_line[0] = piece;
+        s_line[1] = piece_end;
+    }
     {
         // the sequence that holds unit piece_begin, by a block-wide scan over kThreads sequences at a time
         __syncthreads();
         int before = 0; // units of the sequences in front of this pass's
         for (int a0 = 0; a0 < p.n_seqs; a0 += kThreads) {
             const int a = a0 + tid;
-            const int w_a = a < p.n_seqs ? seq_units(p, seq_geom(p, a)) : 0;
+            const int w_a = a < p.n_seqs ? seq_units(p, seq_geom(p, a), whole) : 0;
             int incl = w_a;
 #pragma unroll
             for (int d = 1; d < 32; d <<= 1) {
@@ -368,8 +399,8 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
             const int excl = before + warps_before + incl - w_a;
             if (w_a > 0 && excl <= piece_begin && piece_begin < excl + w_a) {
-                s_sched[2 * kWarps] = a;
-                s_sched[2 * kWarps + 1] = excl;
+                s_sched[3 * kWarps] = a;
+                s_sched[3 * kWarps + 1] = excl;
             }
             before += round_total;
             __syncthreads();
@@ -379,24 +410,25 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
     }
     Walker walker;
-    walker.a = s_sched[2 * kWarps];
-    walker.seq_begin = s_sched[2 * kWarps + 1];
+    walker.a = s_sched[3 * kWarps];
+    walker.seq_begin = s_sched[3 * kWarps + 1];
     walker.g = seq_geom(p, walker.a);
-    walker.n_units = seq_units(p, walker.g);
+    walker.whole = whole;
+    walker.n_units = seq_units(p, walker.g, whole);
     {
         // the last row block that starts at or before the piece: by bisection, a long chunk has hundreds
         int lo = 0, hi = walker.g.n_qb - 1;
         const int at = piece_begin - walker.seq_begin;
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
-            if (units_before(walker.g, mid) * p.nkvh <= at) {
+            if (units_before(walker.g, mid, whole) * p.nkvh <= at) {
                 lo = mid;
             } else {
                 hi = mid - 1;
             }
         }
         walker.qb = lo;
-        walker.qb_begin = units_before(walker.g, lo) * p.nkvh;
+        walker.qb_begin = units_before(walker.g, lo, whole) * p.nkvh;
     }
     {
         Walker first = walker;
@@ -447,16 +479,25 @@ __global__ void __launch_bounds__(kThreads, 1)
     };
     // A warp's place on the line waits in shared memory while its blocks run: a register that is spilled there is fetched from L2 (the
     // operands leave no L1), and a dozen such loads per block cost as much as the block.
-    Place *place = reinterpret_cast<Place *>(s_sched + 32 + warp * kPlaceInts);
-    auto keep_place = [&](const Walker &w, const Fragment &f) {
+    Place *place = reinterpret_cast<Place *>(s_sched + kSchedInts + warp * kPlaceInts);
+    auto keep_place = [&](const Walker &w, const Fragment &f, int pos) {
         __syncwarp();
         if (lane == 0) {
             place->w = w;
             place->f = f;
+            place->pos = pos;
         }
         __syncwarp();
     };
-    keep_place(walker, Fragment{});
+    keep_place(walker, Fragment{}, piece_begin);
+    // The next fragment of the piece, in this warp's place.
+    auto next_fragment = [&](Walker &w, Fragment &f) {
+        int pos = place->pos;
+        w = place->w;
+        const bool found = locate(p, w, pos, s_line[1], f);
+        keep_place(w, f, pos + (found ? f.units : 0));
+        return found;
+    };
 
     // (setmaxnreg inside each branch: where they met again the compiler would keep to the smaller count)
     if (warp >= kProducerWarp) {
@@ -466,13 +507,12 @@ __global__ void __launch_bounds__(kThreads, 1)
             bool alive = true;
             int stage = 0;
             uint32_t turn = 0; // times the ring has been filled
-            for (int pos = piece_begin; alive;) {
+            while (alive) {
                 Fragment f;
-                Walker w = place->w;
-                if (!locate(p, w, pos, piece_end, f)) {
+                Walker w;
+                if (!next_fragment(w, f)) {
                     break;
                 }
-                keep_place(w, f);
                 const int n = f.b1 - f.b0, kept_blocks = w.g.kept_blocks;
                 const int n_pages = (tile_kv_hi(w.g, f.qb) + kPage - 1) / kPage;
                 const int seq_row = (!p.contiguous && p.seq_ids) ? p.seq_ids[f.a] : f.a;
@@ -534,7 +574,6 @@ __global__ void __launch_bounds__(kThreads, 1)
                         }
                     }
                 }
-                pos += n;
             }
             for (int load = max(int(turn) * kStages + stage - kStages, 0); load < int(turn) * kStages + stage; ++load) {
                 drain(kBarFull + load % kStages, uint32_t(load / kStages));
@@ -590,17 +629,15 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
                 __syncwarp();
             };
-            for (int pos = piece_begin;;) {
+            for (;;) {
                 Fragment f;
                 {
-                    Walker w = place->w;
-                    if (!locate(p, w, pos, piece_end, f)) {
+                    Walker w;
+                    if (!next_fragment(w, f)) {
                         break;
                     }
-                    keep_place(w, f);
                 }
                 const int n = __shfl_sync(0xffffffffu, f.b1 - f.b0, 0);
-                pos += n;
                 two = __shfl_sync(0xffffffffu, f.rows, 0) > kHalf;
                 if (h == 1 && !two) { // no rows: see the stages pass (every phase in order) and free them
                     for (int i = 0; i < 2 * n; ++i) {
@@ -693,19 +730,16 @@ __global__ void __launch_bounds__(kThreads, 1)
                 mbar_arrive(bar(kBarEmpty + load % kStages));
             }
         };
-        int pos = piece_begin;
         bool more = false;
-        auto move_on = [&]() { // to the next fragment that has rows for this half: Q rows loaded, place kept
-            Walker w = place->w;
+        auto move_on = [&]() { // to the next fragment that has rows for this half: Q rows loaded
+            Walker w;
             Fragment f;
-            while ((more = locate(p, w, pos, piece_end, f)) && h == 1 && f.rows <= kHalf) {
-                pos += f.b1 - f.b0;
+            while ((more = next_fragment(w, f)) && h == 1 && f.rows <= kHalf) {
                 done += f.b1 - f.b0;
             }
             if (more) {
                 load_q(f, w.g);
             }
-            keep_place(w, f);
         };
         move_on();
         while (more) {
@@ -849,7 +883,6 @@ __global__ void __launch_bounds__(kThreads, 1)
             f = place->f;
             g = place->w.g;
             const int last_load = 2 * (done + n) - 1; // V of the last block
-            pos += n;
             done += n;
             move_on();
             // ---- epilogue of the fragment ---------------------------------------------------------------------------
@@ -860,7 +893,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             const bool whole = f.b0 == 0 && f.b1 == f.tile_nblk;
             bool store_rows = whole;
             float w_own = 1.f, l_all = l, m_all = m_used;
-            const int first_slot = f.tile_begin / piece, last_slot = (f.tile_begin + f.tile_nblk - 1) / piece;
+            const int piece = s_line[0], first_slot = f.tile_begin / piece, last_slot = (f.tile_begin + f.tile_nblk - 1) / piece;
             auto part_of = [&](int s2) { // a fragment's place in the workspace: 1 for the one that begins its tile (and goes on in the next CTA)
                 return p.partials + ((long long)(s2 * 2 + (s2 * piece <= f.tile_begin ? 1 : 0)) * 2 + h) * kPartialFloats;
             };
@@ -887,10 +920,10 @@ __global__ void __launch_bounds__(kThreads, 1)
                     if (last) {
                         p.counters[first_slot * 2 + h] = 0; // ready for the next launch
                     }
-                    s_sched[2 * kWarps + 4 + h] = last ? 1 : 0;
+                    s_sched[3 * kWarps + 2 + h] = last ? 1 : 0;
                 }
                 named_barrier_sync(1 + h, kSoftmaxThreads);
-                store_rows = s_sched[2 * kWarps + 4 + h] != 0;
+                store_rows = s_sched[3 * kWarps + 2 + h] != 0;
                 if (store_rows && !dead) {
                     // weights 2^(m_i - m); sums run over the fragments in the order of their CTAs, this one's terms in its place: the
                     // result does not depend on which fragment happened to arrive last

@@ -776,29 +776,21 @@ def test_kernel_flags_bad_metadata_instead_of_faulting_nvidia(cuda_device):
     assert k_out[3].float().eq(1).all() and not k_out[:3].float().abs().any()
 
 
-@pytest.mark.gpu
-@pytest.mark.parametrize("dname", ["bf16", "f16"])
-@pytest.mark.parametrize("group,nkvh", [(1, 2), (3, 1), (4, 2), (5, 1), (6, 2), (7, 1), (8, 1)])
-@pytest.mark.parametrize("window,keep_first", [(0, 0), (1, 0), (130, 0), (257, 5), (300, 129)])
-def test_prefill_rows_packed_over_the_heads_of_a_group_nvidia(cuda_device, dname, group, nkvh, window, keep_first):
-    """A tile of the chunk kernel is 256 rows of (query, head of the group): chunks that end a row before, at and behind its halves and its
-    end, chunks of one query, of hundreds, with and without context, windows whose edge lies inside a key block and kept first tokens; a
-    scale that turns the order of the scores around. Rounding of the weights and of the result to 16 bits bounds the difference."""
-    d, edge = 128, 256 // group
-    q_lens = [1, edge, max(1, edge // 2), edge + 1, 2 * edge + 3, 700, 1, max(1, 128 // group), 16]
-    before = [0, 0, 129, 127, 1000, 300, 511, 5, 4000]
-    kv_lens = [q + b for q, b in zip(q_lens, before)]
+def check_chunks(dname, group, nkvh, q_lens, before, window=0, keep_first=0, scales=(128 ** -0.5,), num_pages=1000):
+    """Chunks of q_lens queries behind `before` tokens against the float64 statement. Rounding of the weights and of the result to 16 bits
+    bounds the difference."""
+    d, kv_lens = 128, [q + b for q, b in zip(q_lens, before)]
     g = torch.Generator().manual_seed(group * 1000 + window)
     dt = helpers.TORCH_DTYPE[dname]
     ks, vs = ([workloads.randn((n, nkvh, d), dt, g) for n in kv_lens] for _ in range(2))
     q = workloads.randn((sum(q_lens), group * nkvh, d), dt, g)
-    order, counts = torch.randperm(1000, generator=g).tolist(), [-(-n // 16) for n in kv_lens]
+    order, counts = torch.randperm(num_pages, generator=g).tolist(), [-(-n // 16) for n in kv_lens]
     ends = np.cumsum(counts)
-    cache, seqs = helpers.build_cache(NVIDIA, dname, [order[e - n:e] for e, n in zip(ends, counts)], num_pages=1000, nkvh=nkvh, d=d)
+    cache, seqs = helpers.build_cache(NVIDIA, dname, [order[e - n:e] for e, n in zip(ends, counts)], num_pages=num_pages, nkvh=nkvh, d=d)
     helpers.append_all(cache, 0, seqs, ks, vs, NVIDIA)
     i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")  # noqa: E731
     starts = [0, *np.cumsum(q_lens).tolist()]
-    for scale in (d ** -0.5, -0.3 * d ** -0.5):
+    for scale in scales:
         out = torch.zeros_like(q, device="cuda")
         cache.attention_dev(0, out, q.cuda(), i32(seqs), i32(starts), i32(kv_lens), n_seqs=len(seqs), total_q=starts[-1], max_q_len=max(q_lens),
                             max_kv_len=max(kv_lens), nh=group * nkvh, scale=scale, stream=llaisys.context_stream(), window=window,
@@ -807,6 +799,8 @@ def test_prefill_rows_packed_over_the_heads_of_a_group_nvidia(cuda_device, dname
         assert cache.last_kernel() == llaisys.Kernel.PREFILL_TC
         out = out.cpu().double()
         for i, (n, kv) in enumerate(zip(q_lens, kv_lens)):
+            if n == 0:
+                continue
             at, keys = torch.arange(kv - n, kv)[:, None], torch.arange(kv)[None, :]
             hidden = keys > at
             if window:
@@ -815,6 +809,31 @@ def test_prefill_rows_packed_over_the_heads_of_a_group_nvidia(cuda_device, dname
             s = torch.einsum("thd,jhd->htj", q[starts[i]:starts[i + 1]].double(), k) * scale
             want = torch.einsum("htj,jhd->thd", s.masked_fill(hidden, -np.inf).softmax(-1), v)
             assert helpers.max_abs(out[starts[i]:starts[i + 1]], want) <= helpers.MAX_ABS[dname] * max(1.0, want.abs().max().item() / 4), (i, scale)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dname", ["bf16", "f16"])
+@pytest.mark.parametrize("group,nkvh", [(1, 2), (3, 1), (4, 2), (5, 1), (6, 2), (7, 1), (8, 1)])
+@pytest.mark.parametrize("window,keep_first", [(0, 0), (1, 0), (130, 0), (257, 5), (300, 129)])
+def test_prefill_rows_packed_over_the_heads_of_a_group_nvidia(cuda_device, dname, group, nkvh, window, keep_first):
+    """A tile of the chunk kernel is 256 rows of (query, head of the group): chunks that end a row before, at and behind its halves and its
+    end, chunks of one query, of hundreds, with and without context, windows whose edge lies inside a key block and kept first tokens; a
+    scale that turns the order of the scores around. Rounding of the weights and of the result to 16 bits bounds the difference."""
+    edge = 256 // group
+    q_lens = [1, edge, max(1, edge // 2), edge + 1, 2 * edge + 3, 700, 1, max(1, 128 // group), 16]
+    before = [0, 0, 129, 127, 1000, 300, 511, 5, 4000]
+    check_chunks(dname, group, nkvh, q_lens, before, window, keep_first, (128 ** -0.5, -0.3 * 128 ** -0.5))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("group,nkvh,q_lens,before,window", [
+    (6, 2, [100] * 24, [200] * 24, 0),  # as many tiles as CTAs, of three blocks: none is cut
+    (8, 2, [512] * 4, [200] * 4, 0), (4, 8, [200, 1, 256, 0, 77, 130, 5, 90], [200, 0, 300, 4, 10, 128, 511, 90], 0),
+    (2, 8, [1 + i % 40 for i in range(150)], [i % 90 for i in range(150)], 0),  # nine whole tiles a CTA
+    (3, 2, [50 + i for i in range(60)], [300] * 60, 130)])
+def test_chunks_of_short_tiles_are_not_cut_nvidia(cuda_device, group, nkvh, q_lens, before, window):
+    """Calls whose tiles are dealt out whole, one or several to a CTA; sequences without a query among them."""
+    check_chunks("bf16", group, nkvh, q_lens, before, window, num_pages=2000)
 
 
 @pytest.mark.gpu
