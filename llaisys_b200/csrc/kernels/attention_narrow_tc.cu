@@ -1,8 +1,11 @@
-// Causal attention of prompt chunks over keys and values that were expanded from latents into plain tensors of the whole batch, on the
-// 5th-generation tensor cores (tcgen05 + TMEM): K rows of up to 192 dims (two pieces of 64 of the head's own and one that all heads share),
-// V rows of 64 or 128, one K and V head per query head.
+// Chunk attention on the 5th-generation tensor cores (tcgen05 + TMEM) in tiles of 128 rows of ONE query head, two CTAs per SM: the calls that
+// attention_prefill_tc.cu's 256 packed rows serve worse (its rule says which, with both times), and prompt chunks over keys and values
+// that were expanded from latents into plain tensors of the whole batch (K rows of up to 192 dims, two pieces of 64 of the head's own and
+// one that all heads share; V rows of 64 or 128; one K and V head per query head).
 //
-// Roofline: tensor.
+// Roofline: tensor. Algorithmic flops per sequence = 4 * nh * d * sum over chunk rows of visible keys
+//                                                  = 4 * nh * 128 * (L * C + L * (L + 1) / 2)
+// for a chunk of L queries after C cached tokens (QK^T and PV, 2 flops per multiply-add; masked work not counted).
 //
 // Work: a TILE is (sequence, block of 128 chunk rows, query head); it visits its visible keys 64 at a time (a BLOCK:
 // 4 pages). All blocks of all tiles, in the order (sequence, row block, head, key block), form one line that is cut
@@ -19,8 +22,9 @@
 // last piece exit at once.
 //
 // Per CTA: 128 query rows in shared memory per fragment; K/V arrive 64 tokens at a time:
-//   warp 4 (producer)  issues TMA tiles (64 tokens x 64 dims, 128-byte swizzle) into two stages of K and one of V, running ahead across
-//                      fragment boundaries;
+//   warp 4 (producer)  reads the block table (32 entries at a time, a group ahead of use) and issues TMA tiles
+//                      (16 tokens x 64 dims, 128-byte swizzle) into a two-stage K/V ring -- K as [2 dim-halves][64 tokens][128 B], V the same -- running ahead
+//                      across fragment boundaries;
 //   warp 5 (MMA)       one thread issues tcgen05.mma (M 128, K 16, bf16/f16 -> f32):
 //                        S = Q . K^T      N 64, 8 instructions, both operands K-major, accumulator S[buf] in TMEM
 //                        O += P . V       N 128, 4 instructions, P from TMEM (A operand), V MN-major (the page layout
@@ -31,8 +35,9 @@
 //                      first 32 columns of the S buffer they came from, O rescaled in TMEM only when a row's max grew
 //                      by more than 2^8 since the last rescale (the stale max is used consistently for P and the
 //                      sum). After a fragment's last block they also load the next fragment's Q rows.
-// TMEM: 256 columns per CTA: S double-buffered (2 x 64) + O (128). Shared memory: Q 48 KiB + K 2 x 24 KiB + V 16 KiB = 112 KiB, so TWO CTAs
-// share an SM (and its 512 TMEM columns): while one CTA's 128 softmax threads work on a block, the other CTA's MMAs keep the tensor pipe busy.
+// TMEM: 256 columns per CTA: S double-buffered (2 x 64) + O (128). Shared memory: Q 32 KiB + K/V 2 x 32 KiB = 96 KiB (expanded: Q 48 KiB,
+// two stages of K of 24 KiB and one of V of 16 KiB, 112 KiB), so TWO CTAs share an SM (and its 512 TMEM columns): while one CTA's 128 softmax threads work on a block, the other
+// CTA's MMAs keep the tensor pipe busy.
 // What bounds a block (measured with clock64 stamps per role): the thread that issues the MMAs. tcgen05.mma issue keeps
 // pace with execution (8 QK^T instructions take the 300 to 600 clocks the pipe needs for them), so every wait, commit
 // and loop step of that thread is time the pipe idles; a block costs it about 1100 clocks of MMAs and as much again
@@ -41,7 +46,8 @@
 // Synchronisation is mbarriers only (plus one named barrier among the softmax threads around the arrival count);
 // tcgen05.commit arrives on them when the tensor pipe has finished. Barrier phases run on across fragments: stage and
 // parity come from the count of blocks the CTA has done. Every wait is bounded: a wait that runs out sets bit 8 of the
-// error word and the CTA winds down (TMEM is freed, arrival counts stay consistent) instead of hanging.
+// error word; its warp stops and the others stop at their next wait, arrival counts stay consistent, and every role sees its own copies or
+// MMAs done before TMEM is freed.
 // No cluster launch, no multicast.
 #include "kernels.hpp"
 #include "mma_utils.cuh"
@@ -63,6 +69,7 @@ constexpr int kD = 128;
 constexpr int kPage = 16;
 constexpr int kBlockM = 128;                 // query rows per tile
 constexpr int kBlockN = 64;                  // keys per K/V block (4 pages)
+constexpr int kPagesPerBlock = kBlockN / kPage;
 constexpr int kStages = 2;
 constexpr int kSoftmaxThreads = 128;
 constexpr int kProducerWarp = 4, kMmaWarp = 5;
@@ -103,24 +110,36 @@ enum : int {
                                       // earlier, which the MMA thread has waited for)
     kBarPVDone = kBarPFull + 1,       // [2] MMA (commit) -> softmax: O stable; -> producer: V stage is free
     kBarQFull = kBarPVDone + 2,       // softmax (128) -> MMA: Q rows of the next fragment are in shared memory
-    kBarMerge = kBarQFull + 1,        // bulk copy -> softmax: the other half of a split tile is in shared memory
+    kBarDrain = kBarQFull + 1,        // MMA (commit) -> the issuer itself: everything it issued has finished
+    kBarMerge = kBarDrain + 1,        // bulk copy -> softmax: the other half of a split tile is in shared memory
     kNumBars = kBarMerge + 1
 };
 
-struct ExpandedParams {
+struct NarrowParams {
+    long long page0;
+    const int32_t *block_table;
+    int32_t table_stride, num_pages;
+    const int32_t *seq_ids;
     const int32_t *kv_lens;
-    const int32_t *q_starts; // [n_seqs + 1]
-    int32_t n_seqs, nh;
+    const int32_t *q_starts; // [n_seqs + 1]; null in contiguous mode
+    int32_t contiguous;      // 1: K and V are plain [tokens, nkvh, 128] tensors of ONE sequence (no block table, two
+                             // 3-D tensor maps); q rows [0, const_q_len), const_kv_len keys
+    int32_t const_q_len, const_kv_len;
+    int32_t n_seqs, nkvh, group, nh;
     const void *q;
     void *out;
     float scale_log2;
     int32_t *error_flag;
     float *partials;   // [2 * gridDim.x][kPartialFloats]
     int32_t *counters; // [gridDim.x], zero between launches
-    // rows of out lie out_stride elements apart and head h of row r is multiplied by row_scale[r * nh + h] (null: 1)
+    // windowed instantiation: query t sees keys j > t + off - window and j < keep_first; rows of out lie out_stride elements apart and head h
+    // of row r is multiplied by row_scale[r * nh + h] (null: 1)
+    int32_t window, keep_first;
     long long out_stride;
     const float *row_scale;
-    // sequence a's keys are rows 16 page_starts[a] .. of plain tensors (page_starts[a] < 0: not part of the call); a
+    // fading instantiation: fade_a[h] log2(1 + fade_b[h] (distance)) is taken off the scores in the log2 domain
+    const float *fade_a, *fade_b;
+    // expanded instantiation: sequence a's keys are rows 16 page_starts[a] .. of plain tensors (page_starts[a] < 0: not part of the call); a
     // key is nope_halves 64-dim pieces of its own head (from `dim` dims) and one that all heads share (`rot` dims); V rows of dv
     const int32_t *page_starts;
     int32_t dim, rot, dv, nope_halves;
@@ -131,33 +150,57 @@ struct ExpandedParams {
 
 struct SeqGeom {
     int q_start, q_len, kv_len, off, n_qb;
+    int window;      // 0: none
+    int kept_blocks; // 64-key blocks that hold the first tokens a window keeps
 };
 
-__device__ __forceinline__ SeqGeom seq_geom(const ExpandedParams &p, int a) {
+__device__ __forceinline__ SeqGeom seq_geom(const NarrowParams &p, int a) {
     SeqGeom g;
-    g.q_start = p.q_starts[a];
-    g.q_len = p.page_starts[a] < 0 ? 0 : p.q_starts[a + 1] - g.q_start;
-    g.kv_len = max(p.kv_lens[a], g.q_len);
+    if (p.contiguous) {
+        g.q_start = 0;
+        g.q_len = p.const_q_len;
+        g.kv_len = max(p.const_kv_len, g.q_len);
+    } else {
+        g.q_start = p.q_starts[a];
+        g.q_len = p.page_starts != nullptr && p.page_starts[a] < 0 ? 0 : p.q_starts[a + 1] - g.q_start;
+        g.kv_len = min(max(p.kv_lens[a], g.q_len), p.table_stride * kPage);
+    }
+    g.q_len = min(g.q_len, g.kv_len); // (a chunk longer than the tables can hold: flagged elsewhere, never off the end here)
     g.off = g.kv_len - g.q_len; // query t sees keys j <= t + off
     g.n_qb = (g.q_len + kBlockM - 1) / kBlockM;
+    g.window = p.window;
+    g.kept_blocks = (p.keep_first + kBlockN - 1) / kBlockN;
     return g;
 }
 
 // keys any row of row block qb can see, and the 64-key blocks that hold them
 __device__ __forceinline__ int tile_kv_hi(const SeqGeom &g, int qb) { return min(g.kv_len, qb * kBlockM + kBlockM + g.off); }
-__device__ __forceinline__ int tile_blocks(const SeqGeom &g, int qb) { return (tile_kv_hi(g, qb) + kBlockN - 1) / kBlockN; }
+// key blocks that no row of the row block sees, between the blocks of the kept first tokens and the one where the window of
+// the block's first row begins; a tile's blocks are counted without them
+__device__ __forceinline__ int tile_gap(const SeqGeom &g, int qb) {
+    return g.window > 0 ? max(qb * kBlockM + g.off - g.window + 1 - g.kept_blocks * kBlockN, 0) / kBlockN : 0;
+}
+__device__ __forceinline__ int tile_blocks(const SeqGeom &g, int qb) {
+    return (tile_kv_hi(g, qb) + kBlockN - 1) / kBlockN - tile_gap(g, qb);
+}
 
 // units of the line that a sequence takes: per tile its blocks, then kTileCost units that stand for no block
-__device__ __forceinline__ int seq_blocks(const ExpandedParams &p, const SeqGeom &g) {
+__device__ __forceinline__ int seq_blocks(const NarrowParams &p, const SeqGeom &g) {
     // the sum of tile_blocks over the row blocks in closed form (a loop over them, three times per CTA in front of all work,
     // was a large part of a launch over one long chunk): row block qb < n - 1 ends at key (qb + 1) 128 + off, the last one at
-    // kv_len
+    // kv_len; blocks in front of the window are 2 qb + floor((off - window + 1) / 64), less the kept ones, where that is not negative
     static_assert(kBlockM == 2 * kBlockN, "row blocks advance two key blocks");
     const int n = g.n_qb;
     if (n == 0) {
         return 0;
     }
-    const int per_head = (n - 1) * n + (n - 1) * ((g.off + kBlockN - 1) / kBlockN) + (g.kv_len + kBlockN - 1) / kBlockN + n * kTileCost;
+    int per_head = (n - 1) * n + (n - 1) * ((g.off + kBlockN - 1) / kBlockN) + (g.kv_len + kBlockN - 1) / kBlockN + n * kTileCost;
+    if (g.window > 0) {
+        const int a = g.off - g.window + 1 - g.kept_blocks * kBlockN, q0 = a >= 0 ? 0 : (-a + kBlockM - 1) / kBlockM;
+        if (q0 < n) {
+            per_head -= (n - 1) * n - (q0 - 1) * q0 + (n - q0) * (a >> 6); // (an arithmetic shift: floor)
+        }
+    }
     return per_head * p.nh;
 }
 
@@ -173,14 +216,15 @@ struct Walker {
 
 struct Fragment {
     int a, qb, h;
-    int b0, b1;     // key blocks [b0, b1) of the tile
+    int b0, b1;     // key blocks [b0, b1) of the tile, counted without its gap
+    int gap;        // tile_gap
     int tile_nblk;  // blocks of the whole tile
     int tile_begin; // index on the line of the tile's block 0
 };
 
 // The fragment that starts at or after unit `pos` of the line and before piece_end: `pos` moves on to its first block
 // (over the units at a tile's end that stand for no block). False when the piece holds no further block.
-__device__ __forceinline__ bool locate(const ExpandedParams &p, Walker &w, int &pos, int piece_end, Fragment &f) {
+__device__ __forceinline__ bool locate(const NarrowParams &p, Walker &w, int &pos, int piece_end, Fragment &f) {
     while (pos < piece_end) {
         while (pos >= w.seq_begin + w.n_blocks && w.a + 1 < p.n_seqs) {
             w.seq_begin += w.n_blocks;
@@ -212,6 +256,7 @@ __device__ __forceinline__ bool locate(const ExpandedParams &p, Walker &w, int &
         f.h = h;
         f.b0 = b0;
         f.tile_nblk = nb;
+        f.gap = tile_gap(w.g, qb);
         f.b1 = min(nb, b0 + (piece_end - pos));
         f.tile_begin = pos - b0;
         return true;
@@ -250,15 +295,25 @@ __device__ __forceinline__ void add2(float &s0, float &s1, float a0, float a1) {
         : "f"(a0), "f"(a1));
 }
 
-template <bool kBf16>
+// What an instantiation of the kernel adds to plain causal attention; the plain kernel's loops carry nothing of it.
+enum Form {
+    kPlain,
+    kWindowed, // sliding window, output row stride and output factor
+    kFading,   // the same with a distance penalty
+    kExpanded, // output row stride and factor; K and V in plain tensors of the whole batch, K rows of up to 192 in three pieces of 64 dims
+};
+
+template <bool kBf16, int kForm>
 __global__ void __launch_bounds__(kThreads, 2)
-    attention_expanded_tc_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap tmap_v,
-                            const __grid_constant__ CUtensorMap tmap_r, ExpandedParams p) {
-    constexpr int kPieces = 3; // of a Q or K row
+    attention_narrow_tc_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap tmap_v,
+                            const __grid_constant__ CUtensorMap tmap_r, NarrowParams p) {
+    constexpr bool kWin = kForm == kWindowed || kForm == kFading, kFade = kForm == kFading, kWide = kForm == kExpanded, kRows = kForm != kPlain;
+    constexpr int kPieces = kWide ? 3 : 2; // of a Q or K row
     constexpr int kQBytes = kPieces * kQHalfBytes;
-    // two K stages, then ONE stage of V (so that two CTAs fit an SM)
-    constexpr int kKStride = kPieces * kKvHalfBytes, kVAt = 2 * kKStride;
-    static_assert(kVAt + kKvOperandBytes == kStages * kStageBytes, "the ring");
+    // K and V of a stage side by side; expanded: two K stages, then ONE stage of V (so that two CTAs fit an SM)
+    constexpr int kKStride = kWide ? kPieces * kKvHalfBytes : kStageBytes;
+    constexpr int kVAt = kWide ? 2 * kKStride : kKvOperandBytes, kVStride = kWide ? 0 : kStageBytes;
+    static_assert(!kWide || kVAt + kKvOperandBytes == kStages * kStageBytes, "the same ring");
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const uint32_t raw_u32 = smem_u32(smem_raw);
     const uint32_t base_u32 = (raw_u32 + 1023u) & ~1023u; // swizzled operands need 1 KiB alignment
@@ -286,7 +341,9 @@ __global__ void __launch_bounds__(kThreads, 2)
         for (int a = tid; a < p.n_seqs; a += kThreads) {
             const SeqGeom g = seq_geom(p, a);
             mine += seq_blocks(p, g);
-            mine_max = max(mine_max, g.n_qb > 0 ? (g.kv_len + kBlockN - 1) / kBlockN : 0);
+            // (with a window: what a tile can reach, it only sizes the pieces)
+            const int reach = g.window > 0 ? (g.window + kBlockM - 1 + kBlockN - 1) / kBlockN + 1 + g.kept_blocks : 1 << 30;
+            mine_max = max(mine_max, g.n_qb > 0 ? min((g.kv_len + kBlockN - 1) / kBlockN, reach) : 0);
         }
 #pragma unroll
         for (int d = 16; d > 0; d >>= 1) {
@@ -367,29 +424,55 @@ __global__ void __launch_bounds__(kThreads, 2)
         // the stores are volatile asm, which no load may pass, and one round trip per 16 bytes made a fragment
         // boundary cost six blocks' time.
         const char *q_base = static_cast<const char *>(p.q);
-        constexpr int kRow = kPieces * 8, kAtOnce = 8;
-        const int dim = p.dim, head = dim + p.rot;
-        for (int u0 = first; u0 < kBlockM * kRow; u0 += kAtOnce * stride) {
-            uint4 vals[kAtOnce];
+        if constexpr (kWide) {
+            constexpr int kRow = kPieces * 8, kAtOnce = 8;
+            const int dim = p.dim, head = dim + p.rot;
+            for (int u0 = first; u0 < kBlockM * kRow; u0 += kAtOnce * stride) {
+                uint4 vals[kAtOnce];
 #pragma unroll
-            for (int it = 0; it < kAtOnce; ++it) {
-                const int idx = u0 + it * stride, r = idx / kRow, cc = idx - r * kRow, t = f.qb * kBlockM + r;
-                const int piece = cc >> 3, e = (cc & 7) * 8, last = p.nope_halves;
-                const int at = piece == last ? dim + e : piece * 64 + e, end = piece == last ? head : dim;
-                vals[it] = make_uint4(0u, 0u, 0u, 0u);
-                if (idx < kBlockM * kRow && t < g.q_len && piece <= last && at < end) {
-                    vals[it] = *reinterpret_cast<const uint4 *>(q_base + (((long long)(g.q_start + t) * p.nh + f.h) * head + at) * 2);
+                for (int it = 0; it < kAtOnce; ++it) {
+                    const int idx = u0 + it * stride, r = idx / kRow, cc = idx - r * kRow, t = f.qb * kBlockM + r;
+                    const int piece = cc >> 3, e = (cc & 7) * 8, last = p.nope_halves;
+                    const int at = piece == last ? dim + e : piece * 64 + e, end = piece == last ? head : dim;
+                    vals[it] = make_uint4(0u, 0u, 0u, 0u);
+                    if (idx < kBlockM * kRow && t < g.q_len && piece <= last && at < end) {
+                        vals[it] = *reinterpret_cast<const uint4 *>(q_base + (((long long)(g.q_start + t) * p.nh + f.h) * head + at) * 2);
+                    }
+                }
+#pragma unroll
+                for (int it = 0; it < kAtOnce; ++it) {
+                    const int idx = u0 + it * stride, r = idx / kRow, cc = idx - r * kRow;
+                    if (idx < kBlockM * kRow) {
+                        const uint32_t dst = q_u32 + (cc >> 3) * kQHalfBytes + r * 128 + (((cc & 7) ^ (r & 7)) << 4);
+                        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};\n" ::"r"(dst), "r"(vals[it].x), "r"(vals[it].y),
+                                     "r"(vals[it].z), "r"(vals[it].w)
+                                     : "memory");
+                    }
                 }
             }
+            return;
+        }
+        constexpr int kMaxIter = kBlockM * 16 / kSoftmaxThreads; // the fewest threads that call this
+        uint4 vals[kMaxIter];
 #pragma unroll
-            for (int it = 0; it < kAtOnce; ++it) {
-                const int idx = u0 + it * stride, r = idx / kRow, cc = idx - r * kRow;
-                if (idx < kBlockM * kRow) {
-                    const uint32_t dst = q_u32 + (cc >> 3) * kQHalfBytes + r * 128 + (((cc & 7) ^ (r & 7)) << 4);
-                    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};\n" ::"r"(dst), "r"(vals[it].x), "r"(vals[it].y),
-                                 "r"(vals[it].z), "r"(vals[it].w)
-                                 : "memory");
-                }
+        for (int it = 0; it < kMaxIter; ++it) {
+            const int idx = first + it * stride;
+            const int r = idx >> 4, cc = idx & 15;
+            const int t = f.qb * kBlockM + r;
+            vals[it] = make_uint4(0u, 0u, 0u, 0u);
+            if (idx < kBlockM * 16 && t < g.q_len) {
+                vals[it] = *reinterpret_cast<const uint4 *>(q_base + ((long long)(g.q_start + t) * p.nh + f.h) * (kD * 2) + cc * 16);
+            }
+        }
+#pragma unroll
+        for (int it = 0; it < kMaxIter; ++it) {
+            const int idx = first + it * stride;
+            const int r = idx >> 4, cc = idx & 15;
+            if (idx < kBlockM * 16) {
+                const uint32_t dst = q_u32 + (cc >> 3) * kQHalfBytes + r * 128 + (((cc & 7) ^ (r & 7)) << 4);
+                asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};\n" ::"r"(dst), "r"(vals[it].x), "r"(vals[it].y),
+                             "r"(vals[it].z), "r"(vals[it].w)
+                             : "memory");
             }
         }
     };
@@ -432,12 +515,19 @@ __global__ void __launch_bounds__(kThreads, 2)
         atomicOr(p.error_flag, kErrTimeout);
     };
 
-    if (warp == kProducerWarp) {
-        // ================================ producer: TMA tiles of K and V ================================================
+    // For what is on its way in any case: not cut short by another warp's failure.
+    auto drain = [&](int which, uint32_t parity) {
+        if (!mbar_wait_bounded(bar(which), parity & 1u, kMbarWaitLimit)) {
+            give_up();
+        }
+    };
+
+    if (kWide && warp == kProducerWarp) {
+        // ================================ producer, plain tensors ================================================
         // K runs one block ahead of V: its stage is free as soon as the scores of two blocks before are there, the one stage of V
         // when the product of the block before is done.
         bool alive = true;
-        int done = 0;
+        int done = 0, k_loads = 0, v_loads = 0; // (loads: of the CTA so far)
         const uint32_t k_bytes = uint32_t(p.nope_halves + 1) * kKvHalfBytes;
         for (int pos = piece_begin; alive;) {
             Fragment f;
@@ -459,6 +549,7 @@ __global__ void __launch_bounds__(kThreads, 2)
                     tma_load_2d(dst + p.nope_halves * kKvHalfBytes, &tmap_r, 0, token0 + i * kBlockN, full);
                 }
                 __syncwarp();
+                ++k_loads;
                 return true;
             };
             alive = load_k(0);
@@ -472,6 +563,7 @@ __global__ void __launch_bounds__(kThreads, 2)
                     mbar_arrive_expect_tx(bar(kBarVFull), kKvOperandBytes);
                     tma_load_4d(kv_u32 + kVAt, &tmap_v, 0, token0 + i * kBlockN, 0, f.h, bar(kBarVFull));
                 }
+                v_loads += alive ? 1 : 0;
                 __syncwarp();
             }
             pos += n;
@@ -479,6 +571,103 @@ __global__ void __launch_bounds__(kThreads, 2)
         }
         if (!alive && lane == 0) {
             give_up();
+        }
+        for (int load = max(k_loads - kStages, 0); load < k_loads; ++load) {
+            drain(kBarKFull + (load & 1), uint32_t(load >> 1));
+        }
+        if (v_loads > 0) {
+            drain(kBarVFull, uint32_t(v_loads - 1));
+        }
+    } else if (warp == kProducerWarp) {
+        // ================================ producer: TMA tiles of K and V =========================================
+        bool alive = true;
+        int done = 0; // blocks of earlier fragments: ring stage and parity run on across fragments
+        int loads = 0; // of K and V together, in turn
+        for (int pos = piece_begin; alive;) {
+            Fragment f;
+            if (!locate(p, walker, pos, piece_end, f)) {
+                break;
+            }
+            const int n = f.b1 - f.b0;
+            const int n_pages = (tile_kv_hi(walker.g, f.qb) + kPage - 1) / kPage;
+            const int kvh = f.h / p.group;
+            const int seq_row = (!p.contiguous && p.seq_ids) ? p.seq_ids[f.a] : f.a;
+            const long long tbase = (long long)seq_row * p.table_stride;
+            // Page numbers come 8 blocks (32 table entries, one 128-byte load) at a time, and the group after the
+            // current one is requested a whole group early: a table load issued when its block is due costs more than
+            // a block takes (measured: about 1300 clocks between a V tile and the next K tile, on the critical path
+            // of every block).
+            auto key_block = [&](int b) { return kWin && b >= walker.g.kept_blocks ? b + f.gap : b; };
+            auto load_group = [&](int blk0) {
+                const int idx = kWin ? key_block(blk0 + lane / kPagesPerBlock) * kPagesPerBlock + lane % kPagesPerBlock
+                                     : blk0 * kPagesPerBlock + lane;
+                if (p.contiguous) {
+                    return idx; // block b of the tensor is its tokens [64 b, 64 b + 64)
+                }
+                return idx < n_pages ? p.block_table[tbase + idx] : 0;
+            };
+            int group = load_group(f.b0), next_group = load_group(f.b0 + 8);
+            for (int i = 0; i < n && alive; ++i) {
+                const int gi = done + i, st = gi & 1;
+                const int first = key_block(f.b0 + i) * kPagesPerBlock;
+                const int n_pg = min(kPagesPerBlock, n_pages - first);
+                if (i > 0 && (i & 7) == 0) {
+                    group = next_group;
+                    next_group = load_group(f.b0 + i + 8);
+                }
+                int page = __shfl_sync(0xffffffffu, group, (i & 7) * kPagesPerBlock + (lane & (kPagesPerBlock - 1)));
+                if (lane < n_pg && !p.contiguous && (page < 0 || page >= p.num_pages)) {
+                    atomicOr(p.error_flag, kErrBadPage);
+                    page = 0;
+                }
+                const int c3 = int((p.page0 + page) * 2); // K of the page; V is the next index
+                const uint32_t dst = kv_u32 + st * kStageBytes + lane * 2048;
+#pragma unroll
+                for (int is_v = 0; is_v < 2; ++is_v) {
+                    const int full = (is_v ? kBarVFull : kBarKFull) + st, empty = (is_v ? kBarPVDone : kBarQKDone) + st;
+                    if (gi >= kStages && !__all_sync(0xffffffffu, wait_or_abort(bar(empty), uint32_t((gi >> 1) - 1) & 1u, s_abort))) {
+                        if (lane == 0) {
+                            give_up();
+                        }
+                        alive = false;
+                        break;
+                    }
+                    ++loads;
+                    if (lane == 0) {
+                        mbar_arrive_expect_tx(bar(full), uint32_t(n_pg) * 2 * 2048);
+                    }
+                    __syncwarp();
+                    if (lane < n_pg && is_v) {
+                        // V: ONE box per page -- 64 dims x 16 tokens x the 2 halves of the row -- lands as
+                        // [half][16 tokens][128 B], which is what the MN-major B operand of P.V reads 16 keys at a time
+                        // (tokens past the end of a contiguous tensor read as 0)
+                        const uint32_t at = kv_u32 + st * kStageBytes + kKvOperandBytes + lane * (2 * 2048);
+                        if (p.contiguous) {
+                            tma_load_4d(at, &tmap_v, 0, page * kPage, 0, kvh, bar(full));
+                        } else {
+                            tma_load_5d(at, &tmap_v, 0, 0, 0, kvh, c3 + 1, bar(full));
+                        }
+                    } else if (lane < n_pg) {
+                        // K: the K-major B operand of Q.K^T wants the 64 keys of a block side by side in each 64-dim half,
+                        // so a page is two boxes of 64 dims x 16 tokens
+                        const uint32_t lo = dst, hi = lo + kKvHalfBytes; // dims 0-63, dims 64-127
+                        if (p.contiguous) {
+                            // [tokens][kv-heads][128] tensor: box = 64 dims x 1 head x 16 tokens; tokens past the end read as 0
+                            tma_load_3d(lo, &tmap, 0, kvh, page * kPage, bar(full));
+                            tma_load_3d(hi, &tmap, 64, kvh, page * kPage, bar(full));
+                        } else {
+                            tma_load_4d(lo, &tmap, 0, 0, kvh, c3, bar(full));
+                            tma_load_4d(hi, &tmap, 64, 0, kvh, c3, bar(full));
+                        }
+                    }
+                }
+            }
+            pos += n;
+            done += n;
+        }
+        for (int load = max(loads - 2 * kStages, 0); load < loads; ++load) {
+            const int gi = load >> 1;
+            drain(((load & 1) != 0 ? kBarVFull : kBarKFull) + (gi & 1), uint32_t(gi >> 1));
         }
     } else if (warp == kMmaWarp) {
         // ================================ MMA issuer (one thread) =============================================
@@ -489,16 +678,18 @@ __global__ void __launch_bounds__(kThreads, 2)
             bool ok = true;
             auto issue_pv = [&](int gj, bool first_of_fragment) { // O (+)= P . V of the CTA's gj-th block
                 if (!wait_or_abort(bar(kBarPFull), uint32_t(gj) & 1u, s_abort) ||
-                    !wait_or_abort(bar(kBarVFull), uint32_t(gj) & 1u, s_abort)) {
+                    !wait_or_abort(bar(kBarVFull + (kWide ? 0 : gj & 1)), uint32_t(kWide ? gj : gj >> 1) & 1u, s_abort)) {
                     return false;
                 }
                 tc_fence_after();
-                const uint32_t v_u32 = kv_u32 + kVAt;
+                const uint32_t v_u32 = kv_u32 + (gj & 1) * kVStride + kVAt;
 #pragma unroll
                 for (int kk = 0; kk < kBlockN / 16; ++kk) {
-                    // B = 16 keys x 128 dims of V, MN-major: 8-key groups 1 KiB apart, the block's two 64-dim halves 8 KiB apart, 16 keys
-                    // 2 KiB. A = P rows x 16 keys from tensor memory: 8 columns of packed pairs per step, in S buffer gj & 1
-                    const uint64_t b = smem_desc_sw128(v_u32 + kk * 2048, kKvHalfBytes, 1024);
+                    // B = 16 keys (one page) x 128 dims of V, MN-major: 8-key groups 1 KiB apart, the page's two
+                    // 64-dim halves 2 KiB apart, pages 4 KiB apart. A = P rows x 16 keys from tensor memory: 8 columns
+                    // of packed pairs per step, in S buffer gj & 1
+                    // (plain tensors: the block's two halves 8 KiB apart, 16 keys 2 KiB)
+                    const uint64_t b = kWide ? smem_desc_sw128(v_u32 + kk * 2048, kKvHalfBytes, 1024) : smem_desc_sw128(v_u32 + kk * (2 * 2048), 2048, 1024);
                     umma_f16_ts(tmem_o, tmem_base + kColS + (gj & 1) * kBlockN + kk * 8, b, idesc_pv,
                                 (!first_of_fragment || kk > 0) ? 1u : 0u);
                 }
@@ -525,7 +716,7 @@ __global__ void __launch_bounds__(kThreads, 2)
                     const uint32_t k_u32 = kv_u32 + st * kKStride;
 #pragma unroll
                     for (int ks = 0; ks < kPieces * 4; ++ks) {
-                        if ((ks >> 2) > p.nope_halves) {
+                        if (kWide && (ks >> 2) > p.nope_halves) {
                             break;
                         }
                         const uint64_t a = smem_desc_sw128(q_u32 + (ks >> 2) * kQHalfBytes + (ks & 3) * 32, 0, 1024);
@@ -546,13 +737,15 @@ __global__ void __launch_bounds__(kThreads, 2)
             if (!ok) {
                 give_up();
             }
+            umma_commit(bar(kBarDrain));
+            drain(kBarDrain, 0);
         }
     } else {
         // ================================ softmax: one query row per thread =====================================
         const int row = tid;                       // TMEM lane
         const uint32_t lane_base = uint32_t(warp * 32) << 16;
         const uint32_t tmem_o = tmem_base + lane_base + kColO;
-        // A thread whose wait ran out stops computing but keeps walking the fragments, so that the named barrier and
+        // A warp whose wait ran out stops computing but keeps walking the fragments, so that the named barrier and
         // the arrival counts below see all 128 threads every time.
         bool dead = false;
         int done = 0;
@@ -566,33 +759,51 @@ __global__ void __launch_bounds__(kThreads, 2)
             const int t = f.qb * kBlockM + row;        // query index inside the chunk
             const int last_visible = t + g.off;        // keys j <= last_visible (and < kv_len) take part
             float m_used = -INFINITY, l = 0.f;
-            const float to_log2 = p.scale_log2;
+            const float fade_a = kFade ? p.fade_a[f.h] : 0.f, fade_b = kFade ? p.fade_b[f.h] : 0.f;
+            const float to_log2 = kFade ? 1.f : p.scale_log2; // what the scores still have to be multiplied by
             for (int i = 0; i < n && !dead; ++i) {
                 const int gi = done + i, buf = gi & 1;
-                if (!wait_or_abort(bar(kBarQKDone + buf), uint32_t(gi >> 1) & 1u, s_abort)) {
+                if (!__all_sync(0xffffffffu, wait_or_abort(bar(kBarQKDone + buf), uint32_t(gi >> 1) & 1u, s_abort))) {
                     dead = true;
                     break;
                 }
                 tc_fence_after();
                 const uint32_t tmem_s = tmem_base + lane_base + kColS + buf * kBlockN;
-                const int j0 = (f.b0 + i) * kBlockN;
+                const int j0 = (f.b0 + i + (kWin && f.b0 + i >= g.kept_blocks ? f.gap : 0)) * kBlockN;
                 const int n_ok = min(min(last_visible, g.kv_len - 1) - j0 + 1, kBlockN); // visible columns are [0, n_ok)
+                const int n_lo = kWin ? last_visible - p.window + 1 - j0 : 0; // columns below n_lo lie before the row's window,
+                const int n_kept = kWin ? p.keep_first - j0 : 0;              // those below n_kept are seen all the same
                 uint32_t sr[kBlockN / 32][32];
 #pragma unroll
                 for (int c = 0; c < kBlockN / 32; ++c) {
                     tmem_ld32_nowait(tmem_s + c * 32, sr[c]);
                 }
                 tmem_wait_ld();
+                if constexpr (kFade) {
+                    // (distances are exact; those of hidden keys may be negative, whatever comes of them is masked below)
+                    const float d0 = float(last_visible - j0);
+#pragma unroll
+                    for (int c = 0; c < kBlockN / 32; ++c) {
+#pragma unroll
+                        for (int k = 0; k < 32; k += 2) {
+                            float a0, a1, x0, x1;
+                            fma2(a0, a1, d0 - float(c * 32 + k), d0 - float(c * 32 + k + 1), fade_b, 1.f);
+                            fma2(x0, x1, __uint_as_float(sr[c][k]), __uint_as_float(sr[c][k + 1]), p.scale_log2, 0.f);
+                            sr[c][k] = __float_as_uint(fmaf(-fade_a, fast_log2(a0), x0));
+                            sr[c][k + 1] = __float_as_uint(fmaf(-fade_a, fast_log2(a1), x1));
+                        }
+                    }
+                }
                 // Most blocks lie wholly below the diagonal: the whole warp then skips the mask (warp-uniform choice).
                 // Otherwise the hidden scores become -inf and take the same path: 2^(-inf * scale - m) = 0. (A scale
                 // that is not positive takes the slow path further down.)
-                const bool plain = p.scale_log2 > 0.f;
-                if (plain && !__all_sync(0xffffffffu, n_ok >= kBlockN)) {
+                const bool plain = kFade || p.scale_log2 > 0.f;
+                if (plain && !__all_sync(0xffffffffu, n_ok >= kBlockN && (!kWin || n_lo <= 0 || n_kept >= kBlockN))) {
 #pragma unroll
                     for (int c = 0; c < kBlockN / 32; ++c) {
 #pragma unroll
                         for (int k = 0; k < 32; ++k) {
-                            sr[c][k] = c * 32 + k < n_ok ? sr[c][k] : 0xff800000u;
+                            sr[c][k] = c * 32 + k < n_ok && (!kWin || c * 32 + k >= n_lo || c * 32 + k < n_kept) ? sr[c][k] : 0xff800000u;
                         }
                     }
                 }
@@ -616,7 +827,7 @@ __global__ void __launch_bounds__(kThreads, 2)
                     for (int c = 0; c < kBlockN / 32; ++c) {
 #pragma unroll
                         for (int k = 0; k < 32; ++k) {
-                            if (c * 32 + k < n_ok) {
+                            if (c * 32 + k < n_ok && (!kWin || c * 32 + k >= n_lo || c * 32 + k < n_kept)) {
                                 mx8[k & 7] = fmaxf(mx8[k & 7], __uint_as_float(sr[c][k]) * to_log2);
                             }
                         }
@@ -664,8 +875,8 @@ __global__ void __launch_bounds__(kThreads, 2)
 #pragma unroll
                         for (int k = 0; k < 32; k += 2) {
                             const float p0 =
-                                (c * 32 + k < n_ok) ? fast_exp2(fmaf(__uint_as_float(sr[c][k]), to_log2, neg_m)) : 0.f;
-                            const float p1 = (c * 32 + k + 1 < n_ok)
+                                (c * 32 + k < n_ok && (!kWin || c * 32 + k >= n_lo || c * 32 + k < n_kept)) ? fast_exp2(fmaf(__uint_as_float(sr[c][k]), to_log2, neg_m)) : 0.f;
+                            const float p1 = (c * 32 + k + 1 < n_ok && (!kWin || c * 32 + k + 1 >= n_lo || c * 32 + k + 1 < n_kept))
                                                  ? fast_exp2(fmaf(__uint_as_float(sr[c][k + 1]), to_log2, neg_m))
                                                  : 0.f;
                             l0 += p0;
@@ -682,7 +893,7 @@ __global__ void __launch_bounds__(kThreads, 2)
                 // alone on their SM).
                 const bool any_grow = __any_sync(0xffffffffu, grow);
                 if (gi >= 1) {
-                    if (!wait_or_abort(bar(kBarPVDone + ((gi - 1) & 1)), uint32_t((gi - 1) >> 1) & 1u, s_abort)) {
+                    if (!__all_sync(0xffffffffu, wait_or_abort(bar(kBarPVDone + ((gi - 1) & 1)), uint32_t((gi - 1) >> 1) & 1u, s_abort))) {
                         dead = true;
                         break;
                     }
@@ -723,12 +934,13 @@ __global__ void __launch_bounds__(kThreads, 2)
                 }
             }
             // ---- epilogue of the fragment ---------------------------------------------------------------------------
-            if (!dead && !wait_or_abort(bar(kBarPVDone + ((done + n - 1) & 1)), uint32_t((done + n - 1) >> 1) & 1u, s_abort)) {
+            if (!dead && !__all_sync(0xffffffffu, wait_or_abort(bar(kBarPVDone + ((done + n - 1) & 1)), uint32_t((done + n - 1) >> 1) & 1u, s_abort))) {
                 dead = true;
             }
             tc_fence_after();
             const bool whole = f.b0 == 0 && f.b1 == f.tile_nblk;
-            char *out_row = static_cast<char *>(p.out) + (long long)(g.q_start + t) * p.out_stride * 2 + f.h * (p.dv * 2);
+            char *out_row = static_cast<char *>(p.out) + (kRows ? (long long)(g.q_start + t) * p.out_stride * 2 + f.h * ((kWide ? p.dv : kD) * 2)
+                                                               : ((long long)(g.q_start + t) * p.nh + f.h) * (kD * 2));
             bool store_rows = whole, staged = false;
             float w_own = 1.f, l_all = l, m_all = m_used;
             float w_oth[4] = {0.f, 0.f, 0.f, 0.f}; // staged merge: weights of the other fragments, in the order of their CTAs
@@ -799,8 +1011,9 @@ __global__ void __launch_bounds__(kThreads, 2)
                             ++j;
                         }
                     }
-                    if (!dead && !wait_or_abort(bar(kBarMerge), 0u, s_abort)) {
+                    if (dead || !__all_sync(0xffffffffu, wait_or_abort(bar(kBarMerge), 0u, s_abort))) {
                         dead = true;
+                        drain(kBarMerge, 0);
                     }
                     float m_oth[4], l_oth[4];
 #pragma unroll
@@ -857,7 +1070,7 @@ __global__ void __launch_bounds__(kThreads, 2)
             }
             if (store_rows && (staged || !dead)) {
                 float inv = l_all > 0.f ? 1.f / l_all : 0.f;
-                if (p.row_scale != nullptr && t < g.q_len) {
+                if (kRows && p.row_scale != nullptr && t < g.q_len) {
                     inv *= p.row_scale[(long long)(g.q_start + t) * p.nh + f.h];
                 }
 #pragma unroll
@@ -886,8 +1099,9 @@ __global__ void __launch_bounds__(kThreads, 2)
                                 ++j;
                             }
                         }
-                        if (!dead && !wait_or_abort(bar(kBarMerge), uint32_t(c4 / chunks_per_trip) & 1u, s_abort)) {
+                        if (dead || !__all_sync(0xffffffffu, wait_or_abort(bar(kBarMerge), uint32_t(c4 / chunks_per_trip) & 1u, s_abort))) {
                             dead = true;
+                            drain(kBarMerge, uint32_t(c4 / chunks_per_trip));
                         }
                     }
                     if (dead) {
@@ -955,7 +1169,7 @@ __global__ void __launch_bounds__(kThreads, 2)
                             }
                         }
                     }
-                    if (c4 * 32 >= p.dv) {
+                    if (kWide && c4 * 32 >= p.dv) {
                         continue; // (V rows of 64: the other columns are nothing)
                     }
                     if (t < g.q_len && p.out_wide) {
@@ -1011,7 +1225,7 @@ using EncodeTiledFn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_
                                    const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                    CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-EncodeTiledFn expanded_encode_fn() {
+EncodeTiledFn narrow_encode_fn() {
     static EncodeTiledFn fn = [] {
         void *sym = nullptr;
         cudaDriverEntryPointQueryResult res;
@@ -1027,12 +1241,13 @@ EncodeTiledFn expanded_encode_fn() {
 
 // operands + barriers + TMEM-address / abort words + scheduling words; kAlignSlack bytes for the 1 KiB alignment of the
 // operand area (the dynamic window itself starts aligned when the kernel has no static shared memory)
-constexpr size_t kSmemBytes =
-    size_t(kAlignSlack) + 3 * size_t(kQHalfBytes) + kStages * kStageBytes + kNumBars * sizeof(uint64_t) + 8 + 16 * sizeof(int);
-static_assert(2 * (kSmemBytes + 1024) <= 228 * 1024, "two CTAs per SM");
+constexpr size_t smem_bytes(int pieces) {
+    return size_t(kAlignSlack) + size_t(pieces) * kQHalfBytes + kStages * kStageBytes + kNumBars * sizeof(uint64_t) + 8 + 16 * sizeof(int);
+}
+static_assert(2 * (smem_bytes(3) + 1024) <= 228 * 1024, "two CTAs per SM");
 
 // CTAs of the fixed grid: two per SM
-int expanded_slots() {
+int narrow_slots() {
     static int slots[64] = {};
     int dev = 0;
     LLAISYS_CUDA_CHECK(cudaGetDevice(&dev));
@@ -1045,13 +1260,15 @@ int expanded_slots() {
     return n;
 }
 
-template <bool kBf16>
-void launch(cudaStream_t s, const CUtensorMap &tmap, const CUtensorMap &tmap_v, const CUtensorMap &tmap_r, const ExpandedParams &p, int grid) {
+template <bool kBf16, int kForm>
+void launch(cudaStream_t s, const CUtensorMap &tmap, const CUtensorMap &tmap_v, const CUtensorMap &tmap_r, const NarrowParams &p, int grid,
+            bool overlap) {
+    constexpr size_t kSmemBytes = smem_bytes(kForm == kExpanded ? 3 : 2);
     static std::once_flag once[64];
     int dev = 0;
     LLAISYS_CUDA_CHECK(cudaGetDevice(&dev));
     std::call_once(once[dev & 63], [] {
-        LLAISYS_CUDA_CHECK(cudaFuncSetAttribute(attention_expanded_tc_kernel<kBf16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        LLAISYS_CUDA_CHECK(cudaFuncSetAttribute(attention_narrow_tc_kernel<kBf16, kForm>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                 int(kSmemBytes)));
     });
     cudaLaunchConfig_t cfg{};
@@ -1059,10 +1276,68 @@ void launch(cudaStream_t s, const CUtensorMap &tmap, const CUtensorMap &tmap_v, 
     cfg.blockDim = dim3(unsigned(kThreads));
     cfg.dynamicSmemBytes = kSmemBytes;
     cfg.stream = s;
-    LLAISYS_CUDA_CHECK(cudaLaunchKernelEx(&cfg, attention_expanded_tc_kernel<kBf16>, tmap, tmap_v, tmap_r, p));
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = overlap ? 1 : 0;
+    LLAISYS_CUDA_CHECK(cudaLaunchKernelEx(&cfg, attention_narrow_tc_kernel<kBf16, kForm>, tmap, tmap_v, tmap_r, p));
 }
 
 } // namespace
+
+void attention_narrow_tc(stream_t stream, bool bf16, const void *tile_map, const void *v_map, const KVView &kv, const AttnBatch &batch,
+                         const void *q, float scale, const AttnOut &out, const AttnScratch &scratch) {
+    static_assert(2 * kPartialFloats <= 4 * (128 * kD + 2 * 128), "what attention_prefill_tc_scratch asks for covers this kernel");
+    const bool paged = kv.block_table != nullptr;
+    NarrowParams p{};
+    p.page0 = paged ? kv.tma_page0 : 0;
+    p.block_table = kv.block_table;
+    p.table_stride = kv.table_stride;
+    p.num_pages = kv.num_pages;
+    p.seq_ids = batch.seq_ids;
+    p.kv_lens = batch.kv_lens;
+    p.q_starts = batch.q_starts;
+    p.contiguous = paged ? 0 : 1;
+    p.const_q_len = batch.const_q_len;
+    p.const_kv_len = batch.const_kv_len;
+    p.n_seqs = batch.n_seqs;
+    p.nkvh = kv.nkvh;
+    p.group = batch.nh / kv.nkvh;
+    p.nh = batch.nh;
+    p.q = q;
+    p.out = out.out;
+    p.scale_log2 = scale * 1.4426950408889634f;
+    p.error_flag = scratch.error_flag;
+    const bool fading = batch.fade_a != nullptr, windowed = batch.window > 0 || out.row_scale != nullptr || out.row_stride != 0 || fading;
+    p.window = windowed && batch.window <= 0 ? kv.table_stride * kPage : batch.window; // (a factor alone: a window nothing outgrows)
+    p.keep_first = batch.window > 0 ? batch.keep_first : 0;
+    p.out_stride = out.row_stride != 0 ? out.row_stride : (long long)batch.nh * kD;
+    p.row_scale = out.row_scale;
+    p.fade_a = batch.fade_a;
+    p.fade_b = batch.fade_b;
+    p.out_wide = reinterpret_cast<uintptr_t>(out.out) % 32 == 0 && p.out_stride % 16 == 0 ? 1 : 0;
+    p.partials = scratch.partials;
+    p.counters = scratch.counters;
+    CUtensorMap tmap, tmap_v;
+    memcpy(&tmap, tile_map, sizeof(tmap));
+    memcpy(&tmap_v, v_map, sizeof(tmap_v));
+    auto s = static_cast<cudaStream_t>(stream);
+    const int grid = narrow_slots();
+    auto run = [&](auto form) {
+        constexpr int kForm = decltype(form)::value;
+        bf16 ? launch<true, kForm>(s, tmap, tmap_v, tmap, p, grid, kv.overlap_launch)
+             : launch<false, kForm>(s, tmap, tmap_v, tmap, p, grid, kv.overlap_launch);
+    };
+    if (fading) {
+        run(std::integral_constant<int, kFading>{});
+    } else if (windowed) {
+        run(std::integral_constant<int, kWindowed>{});
+    } else {
+        run(std::integral_constant<int, kPlain>{});
+    }
+    check_launch("attention_narrow_tc");
+}
 
 bool attention_expanded_covers(llaisysDataType_t dtype, size_t dim, size_t rot_dim, size_t vdim) {
     return (dtype == LLAISYS_DTYPE_BF16 || dtype == LLAISYS_DTYPE_F16) && dim != 0 && dim <= kD && dim % 8 == 0 && rot_dim != 0 && rot_dim <= 64 &&
@@ -1071,7 +1346,7 @@ bool attention_expanded_covers(llaisysDataType_t dtype, size_t dim, size_t rot_d
 
 int attention_expanded_tc(stream_t stream, llaisysDataType_t dtype, const ExpandedArgs &a, const AttnScratch &scratch) {
     const bool bf16 = dtype == LLAISYS_DTYPE_BF16;
-    const int grid = expanded_slots();
+    const int grid = narrow_slots();
     if (!attention_expanded_covers(dtype, size_t(a.dim), size_t(a.rot_dim), size_t(a.vdim)) || a.n_seqs <= 0 || a.tokens <= 0 ||
         a.tokens >= (int64_t(1) << 31) || a.shared_stride % 8 != 0 || a.out_stride % 8 != 0 || scratch.error_flag == nullptr ||
         scratch.partials == nullptr || scratch.counters == nullptr || scratch.partials_floats < 2 * size_t(grid) * size_t(kPartialFloats) ||
@@ -1083,7 +1358,7 @@ int attention_expanded_tc(stream_t stream, llaisysDataType_t dtype, const Expand
             return -1;
         }
     }
-    EncodeTiledFn encode = expanded_encode_fn();
+    EncodeTiledFn encode = narrow_encode_fn();
     if (encode == nullptr) {
         return -1;
     }
@@ -1106,11 +1381,14 @@ int attention_expanded_tc(stream_t stream, llaisysDataType_t dtype, const Expand
         !map(&tmap_r, a.k_shared, 2, r_dims, r_strides, r_box)) {
         return -1;
     }
-    ExpandedParams p{};
+    NarrowParams p{};
+    p.table_stride = (1 << 30) / kPage; // (no table bounds a sequence)
     p.kv_lens = a.kv_lens;
     p.q_starts = a.q_starts;
     p.page_starts = a.page_starts;
     p.n_seqs = a.n_seqs;
+    p.nkvh = a.nh;
+    p.group = 1;
     p.nh = a.nh;
     p.q = a.q;
     p.out = a.out;
@@ -1126,7 +1404,7 @@ int attention_expanded_tc(stream_t stream, llaisysDataType_t dtype, const Expand
     p.nope_halves = (a.dim + 63) / 64;
     p.out_wide = reinterpret_cast<uintptr_t>(a.out) % 32 == 0 && p.out_stride % 16 == 0 ? 1 : 0;
     auto s = static_cast<cudaStream_t>(stream);
-    bf16 ? launch<true>(s, tmap, tmap_v, tmap_r, p, grid) : launch<false>(s, tmap, tmap_v, tmap_r, p, grid);
+    bf16 ? launch<true, kExpanded>(s, tmap, tmap_v, tmap_r, p, grid, false) : launch<false, kExpanded>(s, tmap, tmap_v, tmap_r, p, grid, false);
     check_launch("attention_expanded_tc");
     return 0;
 }

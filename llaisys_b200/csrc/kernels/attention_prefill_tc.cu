@@ -38,6 +38,7 @@
 
 #include <cuda.h>
 
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 #include <type_traits>
@@ -65,7 +66,7 @@ constexpr int kPartialFloats = kHalf * kD + 2 * kHalf;
 // Merging a partial costs its reader about as much as kMergeCostBlocks blocks; shorter pieces than sqrt(kMergeCostBlocks * longest tile)
 // would spend more on merging than they save.
 constexpr float kMergeCostBlocks = 1.5f;
-constexpr int kMergeCost = 2; // (for a tile in two or three pieces)
+constexpr int kMergeCost = 5; // (of a tile in two or three pieces: eight blocks whole take 2 us less than in pieces of five units, twelve 3 us more)
 // What a tile costs besides its blocks (loading Q, draining the pipeline, storing its rows: about 11500 clocks), in units of a block's time.
 constexpr int kTileCost = 4;
 
@@ -1177,6 +1178,32 @@ bool contiguous_v_map(CUtensorMap *out, const void *base, const KVView &kv, uint
 
 } // namespace
 
+namespace {
+
+// Calls that take less time in tiles of 128 rows of ONE head, two CTAs per SM, blocks of 64 keys (attention_narrow_tc) than in 256 packed
+// rows. Times of both, narrow first.
+bool narrow(const AttnBatch &batch, int nkvh, int sms, bool paged) {
+    const int64_t heads = int64_t(batch.n_seqs) * batch.nh, tiles = heads * ((batch.max_q_len + 127) / 128);
+    const int64_t keys = batch.window > 0 ? std::min<int64_t>(batch.max_kv_len, int64_t(batch.window) + batch.keep_first + batch.max_q_len)
+                                          : batch.max_kv_len;
+    // One block of 64 keys and one tile per SM at most: half of a block here would be padding (64 tokens, 32 / 8 heads, 11.2 and 15.1 us; 128
+    // tokens are 17.5 and 15.3).
+    if (keys <= 64 && tiles <= sms) {
+        return true;
+    }
+    // A head per kv head and up to 128 queries: a tile here fills one half and the SM's other softmax group idles. With more tiles than SMs
+    // that shows (64 chunks of 64 behind 1000, 16 / 16 heads, two layers: 271 and 301; of 64 behind nothing 94 and 122); not between, where
+    // whole tiles of few blocks still win (24 chunks of 32 behind 200, 8 / 8 heads: 60 and 46), unless the waves are many and full.
+    if (batch.nh == nkvh && batch.total_q <= 128 * int64_t(batch.n_seqs) && heads > sms) {
+        return keys <= 64 || keys > 768 || (batch.total_q >= 64 * int64_t(batch.n_seqs) && heads > 2 * int64_t(sms));
+    }
+    // Plain tensors, with no kernel in front whose end hides this kernel's start, and few tiles to spread over the chip: 512 queries x 1000
+    // keys, 12 / 2 heads, 25.5 and 27.8; 256 x 3000 32.9 and 35.5 (x 600 23.6 and 21.8, x 8000 54 and 48, 1024 x 3000 41 and 39.7).
+    return !paged && batch.nh > nkvh && keys > 640 && keys <= 4096 && tiles <= 48;
+}
+
+} // namespace
+
 int attention_prefill_tc(stream_t stream, llaisysDataType_t dtype, const KVView &kv, const AttnBatch &batch,
                          const void *q, float scale, const AttnOut &out, const AttnScratch &scratch) {
     int32_t *error_flag = scratch.error_flag;
@@ -1247,6 +1274,10 @@ int attention_prefill_tc(stream_t stream, llaisysDataType_t dtype, const KVView 
     } else if (!contiguous_kv_map(&tmap, kv.k_base, kv, uint64_t(batch.const_kv_len), bf16) ||
                !contiguous_v_map(&tmap_v, kv.v_base, kv, uint64_t(batch.const_kv_len), bf16)) {
         return -1;
+    }
+    if (narrow(batch, kv.nkvh, grid, paged)) {
+        attention_narrow_tc(stream, bf16, &tmap, &tmap_v, kv, batch, q, scale, out, scratch);
+        return 0;
     }
     auto s = static_cast<cudaStream_t>(stream);
     auto run = [&](auto form) {

@@ -256,6 +256,11 @@ void attention_prefill_tc_scratch(size_t *floats, size_t *counters);
 int make_kv_tile_tensor_map(void *out_256_bytes, void *pool_base, uint64_t total_rows, uint32_t nkvh,
                             llaisysDataType_t dtype);
 
+// The calls of attention_prefill_tc that its kernel for tiles of 128 rows of one head serves better (see its rule): maps of 128 bytes over K
+// and V, everything else checked by attention_prefill_tc.
+void attention_narrow_tc(stream_t stream, bool bf16, const void *tile_map, const void *v_map, const KVView &kv, const AttnBatch &batch,
+                         const void *q, float scale, const AttnOut &out, const AttnScratch &scratch);
+
 // Decode and short chunks over pages of latents (views whose V rows lie in their K rows) on tcgen05: 16-bit, 16-token pages, V parts of up
 // to 512 elements, rows of whole 16-byte pieces of which at most one 64-element piece lies behind the V part's last 128. batch.q_starts may
 // begin anywhere in q and out (rows are absolute; total_q: rows of this call). Returns -1 if the view or shape is not covered, or the

@@ -872,3 +872,13 @@ def test_chunk_waits_that_run_out_are_reported_nvidia(cuda_device):
             assert e.status == Status.KERNEL
         cache.set_wait_limit(1 << 20)
         assert torch.equal(attend(), first), polls
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("group,nkvh,q_lens,before,window", [
+    (6, 2, [64, 1, 17, 40], [0, 5, 30, 0], 0), (4, 8, [64], [0], 0),  # one block of 64 keys
+    (1, 16, [1, 64, 128, 16] * 5, [0, 0, 0, 40] * 5, 0), (1, 16, [100, 128, 33, 7] * 5, [1000, 900, 2000, 1] * 5, 0),  # a head per kv head
+    (1, 16, [300] + [1] * 23, [700] + [790 + i for i in range(23)], 0), (1, 16, [100, 128, 33, 7] * 5, [1000, 900, 2000, 1] * 5, 900)])
+def test_chunks_in_tiles_of_one_head_nvidia(cuda_device, group, nkvh, q_lens, before, window):
+    """The calls that take 128 rows of one head per tile: see the rule in front of attention_prefill_tc."""
+    check_chunks("f16", group, nkvh, q_lens, before, window, num_pages=2000)

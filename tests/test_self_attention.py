@@ -118,6 +118,18 @@ def test_tiles_over_plain_tensors_nvidia(cuda_device, qlen, kvlen, nh, nkvh, d, 
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("qlen,kvlen,nh,nkvh", [(16, 64, 12, 2), (64, 64, 32, 8), (128, 1000, 12, 2), (512, 1000, 12, 2), (129, 4096, 16, 2),
+                                                (129, 4097, 16, 2), (128, 1000, 32, 32)])
+def test_chunk_kernels_over_plain_tensors_nvidia(cuda_device, qlen, kvlen, nh, nkvh):
+    """16-bit calls on both sides of the rule between the two chunk kernels. Rounding of the weights and of the result to bf16."""
+    g = torch.Generator().manual_seed(qlen + kvlen)
+    q, k, v = (workloads.randn((n, h, 128), torch.bfloat16, g) for n, h in ((qlen, nh), (kvlen, nkvh), (kvlen, nkvh)))
+    got = helpers.run_self_attention(q, k, v, 128 ** -0.5, llaisys.DeviceType.NVIDIA, "bf16")
+    f64 = attention.self_attention_f64(q, k, v, 128 ** -0.5)
+    assert helpers.max_abs(got, f64) <= 8e-3 * max(1.0, f64.abs().max().item())
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("bad", [float("inf"), float("nan")])
 @pytest.mark.parametrize("qlen", [3, 96])
 def test_values_behind_the_mask_stay_out_nvidia(cuda_device, qlen, bad):
