@@ -10,6 +10,7 @@
 // of over it, took 68.
 #include "device_utils.cuh"
 #include "kernels.hpp"
+#include "launch_utils.cuh"
 
 #include <cooperative_groups.h>
 
@@ -372,7 +373,7 @@ void dispatch(cudaStream_t s, const TileParams &p, int d) {
     const int blocks = (p.total + (small ? 127 : 63)) / (small ? 128 : 64);
     int splits = 1;
     // (never fewer than four CTAs where there are keys for them: a sum over 1600 keys in one piece is off by 5.7e-7 where four are by 4.9e-7)
-    while (splits < kMostSplits && splits < blocks && (splits < 4 || (small ? few : many) * splits < 148)) {
+    while (splits < kMostSplits && splits < blocks && (splits < 4 || (small ? few : many) * splits < device_sms())) {
         splits *= 2;
     }
     if (d == 128) {

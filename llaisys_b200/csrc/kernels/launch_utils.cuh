@@ -29,6 +29,17 @@ void launch_programmatic(void (*kernel)(KArgs...), dim3 grid, unsigned block, cu
     launch_programmatic_smem(kernel, grid, block, 0, s, std::forward<Args>(args)...);
 }
 
+inline int device_sms() { // SMs of the current device
+    static int sms[64] = {};
+    int dev = 0;
+    LLAISYS_CUDA_CHECK(cudaGetDevice(&dev));
+    int &n = sms[dev & 63];
+    if (n == 0) {
+        LLAISYS_CUDA_CHECK(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
+    }
+    return n;
+}
+
 inline bool aligned16(const void *p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
 
 // body(T{}) with the element type of dtype
