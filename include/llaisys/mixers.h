@@ -291,6 +291,13 @@ struct LlaisysExperts {
 LLAISYS_API int llaisysExpertsDev(llaisysDeviceType_t device_type, int device_id, llaisysDataType_t dtype, const struct LlaisysExperts *args,
                                   llaisysStream_t stream);
 
+/* One row x [k] of 16-bit activations through weight rows of k: h = x, or with gain (NULL: none) x / sqrt(mean(x^2) + eps) * gain rounded to
+ * dtype. form 0: out[i] = weight_i . h for i < n; 1: out[i] += it; 2 (weight [2 n, k], gate rows then up rows): out[i] = up * silu(gate).
+ * What a decoder's single token takes. LLAISYS_E_UNSUPPORTED, with nothing queued, for f32, k not a multiple of 8 or over 12000, pointers that
+ * are not 16-byte aligned and a linear policy other than 0. */
+LLAISYS_API int llaisysLinearRowDev(llaisysDeviceType_t device_type, int device_id, llaisysDataType_t dtype, void *out, const void *x,
+                                    const void *gain, float eps, const void *weight, size_t n, size_t k, int form, llaisysStream_t stream);
+
 #ifdef __cplusplus
 }
 #endif

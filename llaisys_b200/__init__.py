@@ -11,7 +11,7 @@ from .runtime import RuntimeAPI, context_stream, set_context_runtime
 from .tensor import Tensor
 from .ops import Ops
 from .paged_kv import (Kernel, LlaisysError, PagedKVCache, decode_no_alloc, decode_no_alloc_status, experts_dev, gated_delta_dev,
-                       gated_delta_sizes, gated_linear_dev, gated_linear_segment_floats, last_attention_kernel, lse_merge, min_gru_dev,
+                       gated_delta_sizes, gated_linear_dev, gated_linear_segment_floats, last_attention_kernel, linear_row_dev, lse_merge, min_gru_dev,
                        min_gru_scratch_floats, rotary_table_dev, rotary_table_wide_dev, rotate_pairs_dev, state_space_dev,
                        state_space_sizes)
 from . import models
@@ -20,6 +20,6 @@ from .serving import Engine
 __all__ = [
     "RuntimeAPI", "DeviceType", "DataType", "MemcpyKind", "Stream", "Tensor", "Ops", "models", "Engine",
     "PagedKVCache", "lse_merge", "decode_no_alloc", "decode_no_alloc_status", "LlaisysError", "Status", "Kernel",
-    "gated_delta_dev", "gated_delta_sizes", "gated_linear_dev", "gated_linear_segment_floats", "min_gru_dev", "min_gru_scratch_floats", "rotary_table_dev", "rotary_table_wide_dev",
+    "gated_delta_dev", "gated_delta_sizes", "gated_linear_dev", "gated_linear_segment_floats", "linear_row_dev", "min_gru_dev", "min_gru_scratch_floats", "rotary_table_dev", "rotary_table_wide_dev",
     "rotate_pairs_dev", "state_space_dev", "state_space_sizes", "experts_dev", "last_attention_kernel", "context_stream", "set_context_runtime",
 ]

@@ -393,6 +393,29 @@ size_t llaisysMinGruScratchFloats(size_t n_rows, size_t width) {
 #endif
 }
 
+int llaisysLinearRowDev(llaisysDeviceType_t device_type, int device_id, llaisysDataType_t dtype, void *out, const void *x, const void *gain,
+                        float eps, const void *weight, size_t n, size_t k, int form, llaisysStream_t stream) {
+    if (out == nullptr || x == nullptr || weight == nullptr || form < 0 || form > 2) {
+        return bad("linear row: null argument or unknown form");
+    }
+    bool done = false;
+    const int status = guarded([&] {
+#ifdef ENABLE_NVIDIA_API
+        if (device_type == LLAISYS_DEVICE_NVIDIA) {
+            llaisys::core::context().setDevice(device_type, device_id);
+            done = llaisys::kernels::linear_row(stream, dtype, out, x, gain, eps, weight, n, k, static_cast<llaisys::kernels::RowOut>(form));
+        }
+#else
+        (void)device_id, (void)dtype, (void)gain, (void)eps, (void)n, (void)k, (void)stream;
+#endif
+    });
+    if (status == 0 && !done) {
+        llaisys::kernels::set_last_error("linear row: call not covered");
+        return LLAISYS_E_UNSUPPORTED;
+    }
+    return status;
+}
+
 int llaisysMinGruDev(llaisysDeviceType_t device_type, int device_id, llaisysDataType_t dtype, const LlaisysMinGru *a, int decode,
                      llaisysStream_t stream) {
     if (a == nullptr || a->proj == nullptr || a->bias_z == nullptr || a->bias_x == nullptr || a->state == nullptr ||

@@ -31,7 +31,7 @@ struct RowArgs {
 };
 
 template <typename T>
-__global__ void __launch_bounds__(kThreads) linear_row_kernel(RowArgs a) {
+__global__ void __launch_bounds__(kThreads, 2) linear_row_kernel(RowArgs a) {
     extern __shared__ float4 x_s[]; // f(x): the first four elements of every piece, then the last four
     __shared__ float s_norm[kWarps], s_part[kWarps][2];
     const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
@@ -180,7 +180,7 @@ bool linear_row(stream_t stream, llaisysDataType_t dtype, void *out, const void 
     // five warps an SM, so a CTA shares them.
     a.ways = k > 6144 ? kWarps : 1;
     const size_t groups = form == RowOut::kGlu ? n : (n + 1) / 2, per_cta = size_t(kWarps / a.ways);
-    const unsigned grid = unsigned(std::min<size_t>((groups + per_cta - 1) / per_cta, 148 * 2)); // (two CTAs fit an SM)
+    const unsigned grid = unsigned(std::min<size_t>((groups + per_cta - 1) / per_cta, size_t(device_sms()) * 2)); // (two CTAs fit an SM)
     auto s = static_cast<cudaStream_t>(stream);
     if (dtype == LLAISYS_DTYPE_BF16) {
         launch_programmatic_smem(linear_row_kernel<__nv_bfloat16>, grid, kThreads, k * sizeof(float), s, a);

@@ -448,6 +448,8 @@ PROTOTYPES: dict[str, tuple] = {
     "llaisysStateSpaceSizes": (None, [llaisysDataType_t, c_size_t, c_size_t, c_size_t, c_size_t, c_size_t, c_size_t, POINTER(c_size_t),
                                       POINTER(c_size_t), POINTER(c_size_t)]),
     "llaisysExpertsDev": (c_int, [llaisysDeviceType_t, c_int, llaisysDataType_t, POINTER(LlaisysExperts), llaisysStream_t]),
+    "llaisysLinearRowDev": (c_int, [llaisysDeviceType_t, c_int, llaisysDataType_t, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_size_t,
+                                    c_size_t, c_int, llaisysStream_t]),
     "llaisysMinGruDev": (c_int, [llaisysDeviceType_t, c_int, llaisysDataType_t, POINTER(LlaisysMinGru), c_int, llaisysStream_t]),
     "llaisysRotaryTableDev": (c_int, [llaisysDeviceType_t, c_int, c_void_p, c_void_p, c_void_p, c_size_t, c_size_t,
                                       llaisysStream_t]),

@@ -357,6 +357,12 @@ class PagedKVCache:
             _addr(kv_lens_dev), n_seqs, total_q, max_q_len, max_kv_len, nh, scale, window, byref(gates), row_stride, stream))
 
 
+def linear_row_dev(dtype: DataType, out, x, gain, eps: float, weight, n: int, k: int, form: int, *, stream, device_id: int = 0) -> None:
+    """One row of activations through a weight matrix, with the norm in front and the residual add or gate behind (llaisysLinearRowDev)."""
+    _check(LIB_LLAISYS.llaisysLinearRowDev(int(DeviceType.NVIDIA), device_id, int(dtype), _addr(out), _addr(x),
+                                           None if gain is None else _addr(gain), eps, _addr(weight), n, k, form, stream))
+
+
 def min_gru_dev(dtype: DataType, *, decode: bool, stream, device_id: int = 0, **fields) -> None:
     """minGRU on device buffers; fields of LlaisysMinGru (include/llaisys/mixers.h), buffers may be tensors."""
     pointers = {"proj", "bias_z", "bias_x", "state", "seq_ids_dev", "q_starts_dev", "kv_lens_dev", "out", "scratch"}

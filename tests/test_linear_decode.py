@@ -75,3 +75,62 @@ def test_decode_projection_is_deterministic_nvidia(cuda_device):
         outs.append(helpers.tensor_words(helpers.from_llaisys(out, "bf16")))
     llaisys.Ops.set_linear_policy(0)
     assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
+def run_row(dname, form, n, k, gain, offset=0):
+    """One call; what is in `out` afterwards (guard elements behind it included), its start and the float64 statement with a bound on the
+    difference: f32 sums of k products, the norm's rounding of h to 16 bits (one unit, since its f32 value may lie on the other side of a
+    tie) and one rounding of the result."""
+    dt, unit = helpers.TORCH_DTYPE[dname], {"bf16": 2.0 ** -8, "f16": 2.0 ** -11, "f32": 2.0 ** -24}[dname]
+    g = torch.Generator().manual_seed(n + k + form)
+    x = (torch.randn(k, generator=g) * 2).to(dt)
+    scale = (1 + 0.1 * torch.randn(k, generator=g)).to(dt) if gain else None
+    w = (torch.randn((2 * n if form == 2 else n, k), generator=g) * k ** -0.5).to(dt)
+    before = torch.randn(n + 8, generator=g).to(dt)
+    out, dev = before.cuda(), [None if t is None else torch.cat([t.flatten()[:offset], t.flatten()]).cuda()[offset:] for t in (x, scale, w)]
+    torch.cuda.synchronize()
+    try:
+        llaisys.linear_row_dev(helpers.LL_DTYPE[dname], out, dev[0], dev[1], 1e-6, dev[2], n, k, form, stream=llaisys.context_stream())
+        covered = True
+    except llaisys.LlaisysError as e:
+        assert e.status == llaisys.Status.UNSUPPORTED
+        covered = False
+    torch.cuda.synchronize()
+    got = out.cpu()
+    h = x.double()
+    if gain:
+        h = (h / torch.sqrt(h.square().mean() + 1e-6) * scale.double()).to(dt).double()
+    sums, size = w.double() @ h, w.double().abs() @ h.abs()
+    off = size * (k * 2.0 ** -24 + (2 * unit if gain else 0.0))
+    if form == 2:
+        gate, up = sums[:n], sums[n:]
+        want = up * gate * torch.sigmoid(gate)
+        off = off[n:] * (gate.abs() + off[:n]) + 1.1 * off[:n] * up.abs()  # (silu is no larger than its argument and no steeper than 1.1)
+    else:
+        want = sums + (before[:n].double() if form == 1 else 0.0)
+    return covered, got, before, want, off + 1.01 * unit * want.abs() + 1e-6
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dname", ["bf16", "f16"])
+@pytest.mark.parametrize("form,gain", [(0, False), (0, True), (1, False), (2, True)])
+@pytest.mark.parametrize("n,k", [(1, 8), (321, 264), (2048, 1536), (77, 1544), (5001, 2056), (130, 4096), (33, 6144),  # a warp per row pair, 1 to 4 pieces
+                                 (3, 6152), (1301, 8960), (40, 11008), (7, 12000)])  # eight warps per pair, with several pairs a CTA
+def test_row_against_float64_nvidia(cuda_device, dname, form, gain, n, k):
+    covered, got, before, want, bound = run_row(dname, form, n, k, gain)
+    assert covered
+    assert torch.equal(helpers.tensor_words(got[n:]), helpers.tensor_words(before[n:])), "elements behind the output changed"
+    excess = (got[:n].double() - want).abs() - bound
+    assert bool((excess <= 0).all()), excess.max().item()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dname,n,k,offset,policy", [("bf16", 64, 12008, 0, 0), ("bf16", 64, 36, 0, 0), ("f32", 64, 64, 0, 0), ("f16", 64, 64, 1, 0),
+                                                     ("bf16", 64, 64, 0, 2), ("bf16", 64, 64, 0, 1)])
+def test_row_calls_that_are_not_covered_nvidia(cuda_device, dname, n, k, offset, policy):
+    llaisys.Ops.set_linear_policy(policy)
+    try:
+        covered, got, before, _, _ = run_row(dname, 0, n, k, False, offset)
+    finally:
+        llaisys.Ops.set_linear_policy(0)
+    assert not covered and torch.equal(helpers.tensor_words(got), helpers.tensor_words(before))
