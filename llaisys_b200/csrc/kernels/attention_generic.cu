@@ -5,9 +5,10 @@
 // each lane scores one key (a full dot product against the query held in shared memory), the warp folds the 32
 // scores into its running (max, sum) with shuffles, and the P.V update walks the 32 keys with every lane
 // owning head_dim / 32 output dimensions, so V rows are read coalesced. The four warps are merged through
-// shared memory at the end. All arithmetic is f32 with exact expf: this kernel is the on-device statement of
-// the operator's definition (reference: test/ops/self_attention.py:11-28) that the specialised kernels are
-// checked against, and the kernel behind the legacy operator for shapes those do not cover.
+// shared memory at the end. All arithmetic is f32 with exact expf. It stands behind the operator (reference:
+// test/ops/self_attention.py:11-28) and the cache for what no other kernel covers: f32 pools, head dims other than 64
+// and 128, group widths and page sizes the tensor-core kernels do not take. Plain tensors of one sequence with heads of
+// 64 or 128 go to attention_generic_tiles.cu first, from 17 keys on.
 #include "device_utils.cuh"
 #include "kernels.hpp"
 

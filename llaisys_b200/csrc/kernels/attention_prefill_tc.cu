@@ -23,11 +23,11 @@
 //            computed), the accumulator rescaled only when a row's maximum grew by more than 2^8.
 // Tensor memory: 2 x 128 columns of scores, 2 x 128 of accumulators: all 512. Shared memory: Q 64 KiB, ring 160 KiB.
 //
-// The kernel before it ran two CTAs per SM, each with 128 rows and blocks of 64 keys: twice the barriers, commits and TMA boxes per score,
-// and Q K^T at N 64 bound by the shared-memory port. Append and attention of a layer, before and now, many in a row: a prompt of 8192 tokens, 32 / 8 heads 618 and
-// 555 us; 8 chunks of 512 behind up to 8192 tokens, 12 / 2 heads 142 and 130; 24 pieces of 1 to 96 tokens behind up to 3000 55 and 41; 3 of 1500 to
-// 4000 with a window of 1024, 32 / 8 heads 285 and 225. A block takes a CTA about 3000 clocks: a half's chain of scores to registers (250), maximum (350),
-// exponentials (2 x 650) and its MMAs (1024) is what is left above 2048.
+// Tiles of 128 rows of one head on two CTAs per SM (attention_narrow_tc.cu, which took all of these calls before) have twice the barriers,
+// commits and TMA boxes per score, and Q K^T at N 64 bound by the shared-memory port. Append and attention of a layer, narrow and here, many in
+// a row: a prompt of 8192 tokens, 32 / 8 heads 618 and 545 us; 8 chunks of 512 behind up to 8192 tokens, 12 / 2 heads 142 and 127; 24 pieces of
+// 1 to 96 tokens behind up to 3000 55 and 40; 3 of 1500 to 4000 with a window of 1024, 32 / 8 heads 285 and 210. A block takes a CTA about 3000
+// clocks: a half's chain of scores to registers (250), maximum (350), exponentials (2 x 650) and its MMAs (1024) is what is left above 2048.
 //
 // Synchronisation is mbarriers only (and a named barrier per half around the arrival count). Every wait is bounded: one that runs out sets
 // bit 8 of the error word, its lane hands nothing on any more, and the others give up at their next wait. Whatever way a role ends, it sees
@@ -859,8 +859,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                         fma2(x0, x1, __uint_as_float(sr[c][k]), __uint_as_float(sr[c][k + 1]), to_log2, neg_m);
                         const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
                         // With a distance penalty a few near keys dominate a row: there the sum is of the weights as they are multiplied, rounded
-                        // to 16 bits, and the row is off by the rounding of its result alone. (Everywhere it would cost 9 % of a long prompt:
-                        // 604 against 555 us.)
+                        // to 16 bits, and the row is off by the rounding of its result alone. (Everywhere it would cost 9 % of a long prompt.)
                         const uint32_t w = pack2<kBf16>(p0, p1);
                         const float2 r = kFade ? unpack2<kBf16>(w) : make_float2(p0, p1);
                         if (k & 2) {
@@ -1091,7 +1090,7 @@ void launch(cudaStream_t s, const CUtensorMap &tmap, const CUtensorMap &tmap_v, 
 } // namespace
 
 void attention_prefill_tc_scratch(size_t *floats, size_t *counters) {
-    const size_t slots = size_t(chunk_slots()); // (two halves of two fragments per CTA; attention_expanded_tc asks for the same)
+    const size_t slots = size_t(chunk_slots()); // (two halves of two fragments per CTA; attention_narrow_tc.cu needs no more)
     *floats = 4 * slots * size_t(kPartialFloats);
     *counters = 2 * slots;
 }

@@ -7,7 +7,9 @@
 // loads in flight; where K is deep eight warps share two rows. The launch is programmatic and the first loads of W are issued BEFORE the wait
 // for the kernel in front (weights are not written by kernels), so the stream of weights does not stop between the launches of a step; each
 // CTA normalises the row itself. Products and sums are f32, f(x) is rounded to 16 bits as the separate norm rounds it.
-// A prompt of 300 and 24 tokens through four such layers: 8220 -> 6136 us, together with a step that synchronises once instead of three times.
+// One token through four layers and a vocabulary of 32768, steps queued in a row, us before -> now (time of the weights' bytes alone): width 896
+// / 4864 243 -> 193 (30), 1536 / 8960 298 -> 226 (74), 2048 / 5632 345 -> 235 (75), 4096 / 14336 670 -> 508 (312), 5120 / 13824 754 -> 659
+// (393), 8192 / 28672 1504 -> 1423 (1144); depths over kMostK (14336 up) stay with the general path in these.
 #include "launch_utils.cuh"
 #include "mma_utils.cuh"
 
@@ -177,7 +179,7 @@ bool linear_row(stream_t stream, llaisysDataType_t dtype, void *out, const void 
     }
     RowArgs a{out, x, gain, weight, eps, int32_t(n), int32_t(k), 0, form == RowOut::kGlu, form == RowOut::kAdd};
     // Rows of up to 12 KiB go through a warp in a few loads; behind that the few rows of a deep matrix (1536 of 8960) would leave the chip with
-    // five warps an SM, so a CTA shares them.
+    // five warps an SM, so a CTA shares them. (The line was not swept; layers with depths of 5632 to 8192 on either side gain alike, see above.)
     a.ways = k > 6144 ? kWarps : 1;
     const size_t groups = form == RowOut::kGlu ? n : (n + 1) / 2, per_cta = size_t(kWarps / a.ways);
     const unsigned grid = unsigned(std::min<size_t>((groups + per_cta - 1) / per_cta, size_t(device_sms()) * 2)); // (two CTAs fit an SM)
