@@ -8,10 +8,10 @@
 // and a TILE is (sequence, 256 packed rows, kv head). Tiles of 128 queries of one head, as before, filled a chunk of 20 tokens to a sixth
 // and fetched K and V once per head. A tile visits its visible keys 128 at a time (a BLOCK: 8 pages). All blocks of all tiles, in the order
 // (sequence, row block, kv head, key block), form one line that is cut into equal pieces, one per SM, so that every SM gets the same number
-// of blocks whatever the mix of lengths; where tiles are short, whole tiles are dealt out instead. A piece covers the end of one tile, whole tiles, and the beginning of another; each such FRAGMENT
-// runs like a tile. A fragment that is its whole tile normalises and stores its rows; otherwise it stores the accumulator and the rows' (max,
-// sum) into a slot of a workspace and counts itself in, and the fragment that arrives last merges the others with what it holds, in the
-// order of the CTAs and not of arrival. Nobody waits for another CTA.
+// of blocks whatever the mix of lengths; where tiles are short, whole tiles are dealt out instead. A piece covers the end of one tile,
+// whole tiles, and the beginning of another; each such FRAGMENT runs like a tile. A fragment that is its whole tile normalises and stores
+// its rows; otherwise it stores the accumulator and the rows' (max, sum) into a slot of a workspace and counts itself in, and the fragment
+// that arrives last merges the others with what it holds, in the order of the CTAs and not of arrival. Nobody waits for another CTA.
 //
 // Per CTA (one per SM):
 //   warp 8   reads the block table and issues TMA tiles (16 tokens x 64 dims, 128-byte swizzle) into a ring of five 32 KiB stages, K and V of
@@ -30,7 +30,7 @@
 // clocks: a half's chain of scores to registers (250), maximum (350), exponentials (2 x 650) and its MMAs (1024) is what is left above 2048.
 //
 // Synchronisation is mbarriers only (and a named barrier per half around the arrival count). Every wait is bounded: one that runs out sets
-// bit 8 of the error word, its lane hands nothing on any more, and the others give up at their next wait. Whatever way a role ends, it sees
+// bit 8 of the error word, nothing is issued or loaded behind it, and the others give up at their next wait. Whatever way a role ends, it sees
 // its own MMAs or copies done before the CTA gives its tensor memory back and leaves. No cluster launch, no multicast.
 #include "kernels.hpp"
 #include "mma_utils.cuh"
