@@ -1218,8 +1218,8 @@ int run_attention_nvidia(llaisysStream_t stream, llaisysDataType_t dtype, const 
     } else if (fast && out.part == nullptr &&
                (batch.q_starts != nullptr || (view.block_table == nullptr && batch.const_q_len >= 16))) {
         // chunks over a page pool, or the legacy operator's multi-token query over plain K/V tensors from 16 queries on: fewer go
-        // to the f32 tiles behind attention_generic (16 queries x 400 keys, 12 / 2 heads, f32, 14.8 us there; 16 x 300 in bf16 15.4
-        // here). The operator's scratch is sized by the same line.
+        // to the f32 tiles behind attention_generic, in exact f32 (15 queries there and 16 here, 12 / 2 heads: 64 keys 14.9 and 10.8 us,
+        // 1000 keys 14.9 and 23.2, 8000 keys 68 and 35). The operator's scratch is sized by the same line.
         if (kernels::attention_prefill_tc(stream, dtype, view, batch, q, scale, out, scratch) != 0) {
             fail(LLAISYS_E_UNSUPPORTED, "chunk attention (tcgen05 kernel): q, out or K/V are not 16-byte aligned, the pool "
                                         "has no tensor map, or the workspace is missing");
